@@ -24,7 +24,7 @@ template <> struct Phys<ICX_PDE_BURGERS> {
   // F_d = (a_d + b_d u / 2) u - mu_d du/dx_d, mu_0 = mu, mu_1 = mu_t (mu, or 0
   // in spacetime form where the second coordinate is time: a_1 = 1, b_1 = 0
   // give F_t = u, burgers.hpp:261-340)
-  template <class T>
+  template <class T, bool FUSE_E = false>
   __device__ static inline void flux(const PhysParams& pp, const T* u, const T* g, T* F) {
 #pragma unroll
     for (int d = 0; d < 2; ++d) {
@@ -73,8 +73,10 @@ struct NSState {
 constexpr double NS_RGAS = 287.052874;
 
 // Quotients by the density are taken as products with one reciprocal per
-// state (a last-bit difference from dividing each time).
-template <class T>
+// state (a last-bit difference from dividing each time). FUSE_E: the internal
+// energy rhoE / rho - |v|^2 / 2 with one rounding, whatever the compiler
+// would contract (see the base flux of jac_elem_kernel).
+template <class T, bool FUSE_E = false>
 __device__ static inline NSState<T> ns_state(const PhysParams& pp, const T* u) {
   NSState<T> s;
   T gamma = T(pp.gamma);
@@ -87,7 +89,13 @@ __device__ static inline NSState<T> ns_state(const PhysParams& pp, const T* u) {
   s.vv = s.v0 * s.v0 + s.v1 * s.v1;
   s.rhoE = u[3];
   s.E = s.rhoE * s.inv_rho;
-  T e = s.E - T(0.5) * s.vv;
+  T e;
+  if constexpr (FUSE_E) {
+    s.vv = __fmaf_rn(s.v0, s.v0, __fmul_rn(s.v1, s.v1));
+    e = __fmaf_rn(s.rhoE, s.inv_rho, -__fmul_rn(T(0.5), s.vv));
+  } else {
+    e = s.E - T(0.5) * s.vv;
+  }
   s.p = fmax(T(1e-12), (gamma - T(1)) * s.rho * e);
   s.c = sqrt(gamma * s.p * s.inv_rho);
   return s;
@@ -130,9 +138,9 @@ template <> struct Phys<ICX_PDE_NAVIER_STOKES> {
     tau[1][1] -= T(2.0 / 3.0) * mu * div;
   }
 
-  template <class T>
+  template <class T, bool FUSE_E = false>
   __device__ static inline void flux(const PhysParams& pp, const T* u, const T* g, T* F) {
-    NSState<T> s = ns_state(pp, u);
+    NSState<T> s = ns_state<T, FUSE_E>(pp, u);
     T vel[2] = {s.v0, s.v1}, mom[2] = {s.mom0, s.mom1};
     // F[eq*2 + j]
 #pragma unroll
