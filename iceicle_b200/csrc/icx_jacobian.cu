@@ -526,7 +526,7 @@ __global__ void __launch_bounds__((JacCfg<PDE, P, G, T>::THREADS), (JacCfg<PDE, 
       }
     }
     __syncthreads();
-    // over q0, and the lifted faces; the (i0, j0) entries of one (ie, i1, j1, je) per thread
+    // the lifted faces, and over q0; the (i0, j0) entries of one (ie, i1, j1, je) per thread
     for (int t = tid; t < SQ; t += NT) {
       const int je = t % NEQ, j1 = t / NEQ % N1, i1 = t / ROW % N1, ie = ie0 + t / (ROW * N1);
       T acc[N1][N1];
@@ -534,18 +534,6 @@ __global__ void __launch_bounds__((JacCfg<PDE, P, G, T>::THREADS), (JacCfg<PDE, 
       for (int i0 = 0; i0 < N1; ++i0)
 #pragma unroll
         for (int j0 = 0; j0 < N1; ++j0) acc[i0][j0] = T(0.0);
-#pragma unroll
-      for (int q0 = 0; q0 < Q1; ++q0) {
-        const T* S = sm + J::O_S + q0 * SQ + t;
-        const T s0 = S[0], s1 = S[Q1 * SQ], s2 = S[2 * Q1 * SQ], s3 = S[3 * Q1 * SQ];
-#pragma unroll
-        for (int j0 = 0; j0 < N1; ++j0) {
-          const T b = sb[q0 * N1 + j0], db = sdb[q0 * N1 + j0];
-          const T pv = b * s0 + db * s1, qv = b * s2 + db * s3;
-#pragma unroll
-          for (int i0 = 0; i0 < N1; ++i0) acc[i0][j0] += sdb[q0 * N1 + i0] * pv + sb[q0 * N1 + i0] * qv;
-        }
-      }
 #pragma unroll
       for (int lf = 0; lf < 4; ++lf) {
         const T* L = sm + J::O_DFQ + (lf * NQF * NEQ + ie) * BS + j1 * NEQ + je;
@@ -561,6 +549,18 @@ __global__ void __launch_bounds__((JacCfg<PDE, P, G, T>::THREADS), (JacCfg<PDE, 
 #pragma unroll
             for (int i0 = 0; i0 < N1; ++i0) acc[i0][j0] += fx * L[i0 * NEQ * BS + j0 * ROW];
           }
+        }
+      }
+#pragma unroll
+      for (int q0 = 0; q0 < Q1; ++q0) {
+        const T* S = sm + J::O_S + q0 * SQ + t;
+        const T s0 = S[0], s1 = S[Q1 * SQ], s2 = S[2 * Q1 * SQ], s3 = S[3 * Q1 * SQ];
+#pragma unroll
+        for (int j0 = 0; j0 < N1; ++j0) {
+          const T b = sb[q0 * N1 + j0], db = sdb[q0 * N1 + j0];
+          const T pv = b * s0 + db * s1, qv = b * s2 + db * s3;
+#pragma unroll
+          for (int i0 = 0; i0 < N1; ++i0) acc[i0][j0] += sdb[q0 * N1 + i0] * pv + sb[q0 * N1 + i0] * qv;
         }
       }
 #pragma unroll
