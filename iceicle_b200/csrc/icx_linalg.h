@@ -48,6 +48,39 @@ cudaError_t la_tri_rows_f32(const DeviceMesh& dm, bool lower, const float* A, co
                             double sign, double* y, cudaStream_t s);
 cudaError_t la_block_diag_apply(int E, int bs, const double* D, const double* x, double* y, cudaStream_t s);
 // z = y + D y, D block diagonal in FP32 (FP32 accumulation)
+// the apply on whole structured grids by strips of rows (icx_ilu_strip.cu): the
+// grids' strips (elements e0.. and blocks b0.. of an nx x ny grid in natural
+// order on the 5-point pattern; rows j0 .. j0 + nr - 1) and the exchange rows
+// between them, ex[w] the offset of a strip's last row of sweep w (0 forward,
+// 1 backward), which la_ilu_strip_reset prepares once and after a failed apply
+struct IluStrip {
+  int e0, b0, nx, ny, j0, nr;
+  long long ex[2];
+  long long pk;                // byte offset of the strip's packed factors (of the plan's precision)
+};
+struct IluStripPlan {
+  int nstrips = 0;
+  int max_steps = 0, max_nx = 0;  // most steps and widest row of a strip
+  IluStrip* strips = nullptr;  // [nstrips], a grid's strips in ascending order
+  double* ex = nullptr;        // [nex], shared by both precisions' plans
+  long long nex = 0;
+  long long bytes = 0;         // packed factors
+};
+// rows per strip for a block size (0: no strip kernel for it)
+constexpr int ilu_strip_rows(int bs) { return bs <= 4 ? 8 : bs <= 9 ? 4 : bs <= 16 ? 4 : bs <= 25 ? 2 : bs <= 36 ? 1 : 0; }
+// bytes of the packed factors of a strip of nr rows of nx elements
+long long ilu_strip_bytes(int bs, int nx, int nr, bool f32);
+cudaError_t la_ilu_strip_reset(const IluStripPlan& p, cudaStream_t s);
+// the factors (FP64) packed in the order of the strips' steps, once per factorisation
+cudaError_t la_ilu_strip_pack(int bs, const IluStripPlan& p, const double* LU, const double* Uinv, double* pk,
+                              cudaStream_t s);
+cudaError_t la_ilu_strip_pack_f32(int bs, const IluStripPlan& p, const double* LU, const double* Uinv, float* pk,
+                                  cudaStream_t s);
+// y = (LU)^-1 x; f = n doubles of scratch; *err = 1 if a wait ran out
+cudaError_t la_ilu_apply_strips(int bs, const IluStripPlan& p, const double* pk, const double* x, double* y, double* f,
+                                int* err, cudaStream_t s);
+cudaError_t la_ilu_apply_strips_f32(int bs, const IluStripPlan& p, const float* pk, const double* x, double* y,
+                                    double* f, int* err, cudaStream_t s);
 cudaError_t la_block_diag_correct_f32(int E, int bs, const float* D, const double* y, double* z, cudaStream_t s);
 // *d_out = x . y (device scalar, overwritten)
 cudaError_t la_dot_to(long long n, const double* x, const double* y, double* d_out, cudaStream_t s);

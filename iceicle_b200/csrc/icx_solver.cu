@@ -96,6 +96,12 @@ struct icx_solver_work {
   int schedule = 0;         // 0 / 1: data flow (the solvers' apply), 2: rows (icx_ilu_apply only)
   unsigned* cnt_rows = nullptr;
   unsigned epoch_rows = 0;
+  // row strips of the grids for the FP64 and FP32 whole-grid applies (nstrips 0: not natural-order 5-point grids,
+  // or no kernel for the block size), the factors packed for them (allocated on first use) and whether they
+  // hold the current factorisation
+  icx::IluStripPlan sp[2];
+  void* spk[2] = {nullptr, nullptr};
+  bool sp_ok[2] = {false, false};
   IluTilePlan tp;           // tiled block-ILU(0) pattern and schedule (tp.tile == c->ilu_tile once built)
   int* pc_err = nullptr;    // set by the ILU apply if a dependency wait timed out
   double* dh = nullptr;     // device scalars (dot results)
@@ -130,6 +136,8 @@ icx_status set_err(icx_ctx* c, icx_status st, const std::string& m) {
     if (_e != cudaSuccess) return set_err(c, ICX_ERR_CUDA, std::string(#expr) + ": " + \
                                                               cudaGetErrorString(_e)); \
   } while (0)
+
+icx_status build_strip_plan(icx_ctx* c);
 
 icx_status ensure_work(icx_ctx* c, int m) {
   const icx::DeviceMesh& dm = c->dm;
@@ -192,6 +200,72 @@ icx_status ensure_work(icx_ctx* c, int m) {
     }
     w->rows_ok = ok;
   }
+  return build_strip_plan(c);
+}
+
+// the row strips of the whole-grid apply where every grid of the context (the
+// context's own, or each part's of a batch) is stored in natural order on the
+// 5-point element pattern; otherwise the plan stays empty
+icx_status build_strip_plan(icx_ctx* c) {
+  icx_solver_work* w = c->sw;
+  const icx::DeviceMesh& dm = c->dm;
+  const int S = icx::ilu_strip_rows(w->bs);
+  if (S < 1) return ICX_OK;
+  std::vector<std::pair<int, int>> grids;
+  if (c->parts.empty()) grids.push_back({c->nx, c->ny});
+  else
+    for (const icx_ctx* q : c->parts) grids.push_back({q->nx, q->ny});
+  long long total = 0;
+  for (const auto& g : grids) {
+    if (g.first < 1 || g.second < 1) return ICX_OK;
+    total += (long long)g.first * g.second;
+  }
+  if (total != dm.E) return ICX_OK;
+  std::vector<int> rp(dm.E + 1), ci(dm.nnzb);
+  CK(cudaMemcpy(rp.data(), dm.bsr_rowptr, sizeof(int) * rp.size(), cudaMemcpyDeviceToHost));
+  CK(cudaMemcpy(ci.data(), dm.bsr_colidx, sizeof(int) * ci.size(), cudaMemcpyDeviceToHost));
+  std::vector<icx::IluStrip> strips;
+  long long nex = 0;
+  int e0 = 0;
+  for (const auto& g : grids) {
+    const int nx = g.first, ny = g.second, b0 = rp[e0];
+    int at = b0;
+    for (int j = 0; j < ny; ++j)
+      for (int i = 0; i < nx; ++i) {
+        const int e = e0 + j * nx + i;
+        if (rp[e] != at) return ICX_OK;
+        const int want[5] = {j > 0 ? e - nx : -1, i > 0 ? e - 1 : -1, e, i < nx - 1 ? e + 1 : -1,
+                             j < ny - 1 ? e + nx : -1};
+        for (int k : want)
+          if (k >= 0 && (at >= rp[e + 1] || ci[at++] != k)) return ICX_OK;
+        if (at != rp[e + 1]) return ICX_OK;
+      }
+    for (int j = 0; j < ny; j += S) {
+      icx::IluStrip s{e0, b0, nx, ny, j, std::min(S, ny - j), {nex, nex + (long long)nx * w->bs}, 0};
+      nex += 2ll * nx * w->bs;
+      strips.push_back(s);
+    }
+    e0 += nx * ny;
+  }
+  double* ex = nullptr;
+  CK(cudaMalloc((void**)&ex, sizeof(double) * nex));
+  w->sp[0].ex = w->sp[1].ex = ex;
+  for (int pi = 0; pi < 2; ++pi) {
+    icx::IluStripPlan& sp = w->sp[pi];
+    sp.nex = nex;
+    for (icx::IluStrip& s : strips) {
+      s.pk = sp.bytes;
+      sp.bytes += icx::ilu_strip_bytes(w->bs, s.nx, s.nr, pi == 1);
+      sp.max_steps = std::max(sp.max_steps, s.nx + s.nr - 1);
+      sp.max_nx = std::max(sp.max_nx, s.nx);
+    }
+    CK(cudaMalloc((void**)&sp.strips, sizeof(icx::IluStrip) * strips.size()));
+    CK(cudaMemcpy(sp.strips, strips.data(), sizeof(icx::IluStrip) * strips.size(), cudaMemcpyHostToDevice));
+  }
+  CK(icx::la_ilu_strip_reset(w->sp[0], 0));
+  CK(cudaStreamSynchronize(0));
+  // blockIdx.y of the packing kernel counts both sweeps' steps
+  if (2 * w->sp[0].max_steps <= 65535) w->sp[0].nstrips = w->sp[1].nstrips = (int)strips.size();
   return ICX_OK;
 }
 
@@ -393,6 +467,17 @@ cudaError_t tri_rows(icx_ctx* c, bool mixed, bool lower, const double* v, const 
                : icx::la_tri_rows(dm, lower, w->pc, v, x0, -1.0, y, s);
 }
 
+// whether the current launch shape leaves the block-ILU(0) apply to the row strips: whole grids, the sentinel
+// schedule and the default rows per task and CTAs per SM of the data-flow apply
+bool strip_shape(const icx_ctx* c, bool mixed) {
+  const icx_solver_work* w = c->sw;
+  const icx::TileChoice& t = c->dm.tile;
+  const int pi = mixed ? 1 : 0;
+  return !w->tp.tile && w->sp[pi].nstrips > 0 && icx::flow_sentinel(t, pi) &&
+         (t.flow_rows[pi] == 0 || t.flow_rows[pi] == icx::flow_rows_default(w->bs)) &&
+         (t.flow_ctas[pi] == 0 || t.flow_ctas[pi] == 2);
+}
+
 // the data-flow block-ILU(0) apply with the context's launch shape. Each
 // apply adds an element's task count to its counters and waits for
 // epoch x task count, so a change of rows per task (FP64 and FP32 applies may
@@ -425,6 +510,15 @@ cudaError_t ilu_flow(icx_ctx* c, bool mixed, const double* x, double* z, cudaStr
   }
   // the sentinel schedule uses neither the counters nor the epoch
   const bool sen = icx::flow_sentinel(dm.tile, pi);
+  // whole structured grids at the default launch shape: by strips of grid rows
+  // (a level costs a step inside a CTA instead of a trip through L2; a tuned
+  // shape of the data-flow apply, same results, replaces it where it is faster)
+  if (w->sp_ok[pi] && strip_shape(c, mixed)) {
+    const cudaError_t e =
+        mixed ? icx::la_ilu_apply_strips_f32(w->bs, w->sp[1], (const float*)w->spk[1], x, z, w->pct, w->pc_err, s)
+              : icx::la_ilu_apply_strips(w->bs, w->sp[0], (const double*)w->spk[0], x, z, w->pct, w->pc_err, s);
+    if (e != cudaErrorNotSupported) return e;  // not ahead at this size: the data-flow apply, same results
+  }
   if (!sen && rows != w->flow_rows) {
     cudaError_t e = cudaMemsetAsync(w->cnt, 0, sizeof(unsigned) * 2 * dm.E, s);
     if (e != cudaSuccess) return e;
@@ -523,6 +617,16 @@ cudaError_t build_pc_impl(icx_ctx* c, int kind, bool mixed, cudaStream_t s) {
       if (e == cudaSuccess) e = icx::la_ilu_factor(dm, w->order, w->lvl_off, w->pc, w->uinv, w->flag, s);
     }
   }
+  // the strips' packed factors (kind 4 applies its factors by other kernels)
+  w->sp_ok[0] = w->sp_ok[1] = false;
+  const int pi = mixed ? 1 : 0;
+  if (e == cudaSuccess && ilu && kind != 4 && strip_shape(c, mixed)) {
+    if (!w->spk[pi]) e = cudaMalloc(&w->spk[pi], (size_t)w->sp[pi].bytes);
+    if (e == cudaSuccess)
+      e = mixed ? icx::la_ilu_strip_pack_f32(w->bs, w->sp[1], w->pc, w->uinv, (float*)w->spk[1], s)
+                : icx::la_ilu_strip_pack(w->bs, w->sp[0], w->pc, w->uinv, (double*)w->spk[0], s);
+    w->sp_ok[pi] = e == cudaSuccess;
+  }
   if (e != cudaSuccess || !mixed) return e;
   e = icx::la_d2f(nv, w->vals, w->vals32, s);
   if (e == cudaSuccess && jac) e = icx::la_d2f(nd, w->pc, w->pc32, s);
@@ -607,7 +711,7 @@ icx_status gmres(icx_ctx* c, int pc, bool mixed, int m, int maxit, double rtol, 
                         (long long)(uintptr_t)dm.bsr_colidx, (long long)(uintptr_t)dm.bsr_diag,
                         (long long)(uintptr_t)w->order, (long long)w->tp.tile, (long long)(uintptr_t)w->tp.order,
                         (long long)w->fd_on, (long long)(uintptr_t)w->fd_u, (long long)(uintptr_t)w->fd_r,
-                        (long long)w->bf16, (long long)w->cgs_passes})
+                        (long long)w->bf16, (long long)w->cgs_passes, (long long)w->sp_ok[pi]})
       key = (key ^ (unsigned long long)v) * 1099511628211ull;
     kb.graphs = &w->graphs;
     kb.graph_key = key | 1;
@@ -628,6 +732,7 @@ icx_status gmres(icx_ctx* c, int pc, bool mixed, int m, int maxit, double rtol, 
     cudaMemsetAsync(w->pc_err, 0, sizeof(int), s);
     cudaMemsetAsync(w->cnt, 0, sizeof(unsigned) * 2 * dm.E, s);
     cudaMemsetAsync(w->cnt_rows, 0, sizeof(unsigned) * 2 * dm.E, s);
+    icx::la_ilu_strip_reset(w->sp[0], s);
     w->epoch = 0;
     w->epoch_rows = 0;
     return set_err(c, ICX_ERR_CUDA, perr == 2 ? "block-ILU apply: block index out of range"
@@ -709,7 +814,7 @@ void free_solver_work(icx_ctx* c) {
   icx_solver_work* w = c->sw;
   void* ptrs[] = {w->pc16, w->uinv16, w->V32, w->vt, w->vals32, w->pc32, w->uinv32, w->vals, w->pc, w->uinv, w->V, w->w, w->z, w->r, w->res, w->du,
                   w->ustep, w->rwork, w->pct, w->pct2, w->pct3, w->pct4, w->order, w->cnt, w->cnt_rows, w->pc_err,
-                  w->dh, w->flag, w->lw.partial};
+                  w->dh, w->flag, w->lw.partial, w->sp[0].strips, w->sp[1].strips, w->sp[0].ex, w->spk[0], w->spk[1]};
   w->graphs.release();
   for (void* p : ptrs)
     if (p) cudaFree(p);
@@ -891,6 +996,7 @@ icx_status icx_ilu_apply(icx_ctx* c, const double* d_vals, const double* d_x, do
     cudaMemsetAsync(w->pc_err, 0, sizeof(int), s);
     cudaMemsetAsync(w->cnt, 0, sizeof(unsigned) * 2 * c->dm.E, s);
     cudaMemsetAsync(w->cnt_rows, 0, sizeof(unsigned) * 2 * c->dm.E, s);
+    icx::la_ilu_strip_reset(w->sp[0], s);
     w->epoch = 0;
     w->epoch_rows = 0;
     return set_err(c, ICX_ERR_CUDA, perr == 2 ? "block-ILU apply: block index out of range"
@@ -1249,7 +1355,7 @@ unsigned long long solver_graph_key(icx_ctx* c, int pc, bool mixed) {
                       (long long)t.flow_ctas[pi], (long long)t.flow_sched[pi], (long long)(uintptr_t)dm.bsr_rowptr,
                       (long long)(uintptr_t)dm.bsr_colidx, (long long)(uintptr_t)dm.bsr_diag,
                       (long long)(uintptr_t)w->order, (long long)w->tp.tile, (long long)(uintptr_t)w->tp.order,
-                      (long long)(uintptr_t)w->vals, (long long)(uintptr_t)w->pc})
+                      (long long)(uintptr_t)w->vals, (long long)(uintptr_t)w->pc, (long long)w->sp_ok[pi]})
     key = (key ^ (unsigned long long)v) * 1099511628211ull;
   return key;
 }
@@ -1270,6 +1376,7 @@ icx_status solver_take_pc_err(icx_ctx* c, int* err) {
     // the counters are inconsistent after an abandoned apply: start over
     CK(cudaMemsetAsync(w->pc_err, 0, sizeof(int), s));
     CK(cudaMemsetAsync(w->cnt, 0, sizeof(unsigned) * 2 * c->dm.E, s));
+    CK(icx::la_ilu_strip_reset(w->sp[0], s));
     w->epoch = 0;
     CK(cudaStreamSynchronize(s));
   }
