@@ -57,139 +57,541 @@ __device__ inline int find_block(const int* rowptr, const int* colidx, int r, in
 }
 
 // C = X Y for BS x BS blocks in shared memory, each thread owning 4 x 4
-// output tiles; op(tile, r0, c0, acc) consumes every finished tile
-template <int BS, class Op>
-__device__ inline void block_gemm(const double* X, const double* Y, Op op) {
-  constexpr int NT = (BS + 3) / 4;
-  for (int tt = threadIdx.x; tt < NT * NT; tt += blockDim.x) {
-    const int r0 = (tt / NT) * 4, c0 = (tt % NT) * 4;
-    double acc[4][4];
+// output tiles; op(r0, c0, acc) consumes every finished tile
+template <int BS>
+__device__ inline void block_gemm_tile(const double* X, const double* Y, int r0, int c0, double (&acc)[4][4]) {
+#pragma unroll
+  for (int a = 0; a < 4; ++a)
+#pragma unroll
+    for (int b = 0; b < 4; ++b) acc[a][b] = 0.0;
+  for (int m = 0; m < BS; ++m) {
+    double xa[4], yb[4];
+#pragma unroll
+    for (int a = 0; a < 4; ++a) xa[a] = (r0 + a < BS) ? X[(r0 + a) * BS + m] : 0.0;
+#pragma unroll
+    for (int b = 0; b < 4; ++b) yb[b] = (c0 + b < BS) ? Y[m * BS + c0 + b] : 0.0;
 #pragma unroll
     for (int a = 0; a < 4; ++a)
 #pragma unroll
-      for (int b = 0; b < 4; ++b) acc[a][b] = 0.0;
-    for (int m = 0; m < BS; ++m) {
-      double xa[4], yb[4];
-#pragma unroll
-      for (int a = 0; a < 4; ++a) xa[a] = (r0 + a < BS) ? X[(r0 + a) * BS + m] : 0.0;
-      if (BS % 4 == 0) {
-        const double2* y2 = reinterpret_cast<const double2*>(Y + m * BS + c0);
-        double2 u0 = y2[0], u1 = y2[1];
-        yb[0] = u0.x; yb[1] = u0.y; yb[2] = u1.x; yb[3] = u1.y;
-      } else {
-#pragma unroll
-        for (int b = 0; b < 4; ++b) yb[b] = (c0 + b < BS) ? Y[m * BS + c0 + b] : 0.0;
-      }
-#pragma unroll
-      for (int a = 0; a < 4; ++a)
-#pragma unroll
-        for (int b = 0; b < 4; ++b) acc[a][b] += xa[a] * yb[b];
-    }
-    op(r0, c0, acc);
+      for (int b = 0; b < 4; ++b) acc[a][b] += xa[a] * yb[b];
   }
 }
 
+// Shapes of the row factorisation and of the block products. Blocks whose size
+// is a multiple of 4 (above 4) go through the FP64 matrix instructions
+// (8 x 8 x 4): warp w owns rows 8 w .. 8 w + 7 of the result, lane l rows l / 4
+// and column pairs 8 t + 2 (l % 4); staged blocks have rows of LD doubles, LD * 8
+// bytes = 32 modulo 128, so that neither operand's fragments conflict in shared
+// memory. Odd sizes keep a 4 x 4 tile per thread. The rate of the FP64 pipe is
+// the same either way (64 multiply-adds per clock and SM); what the matrix form
+// saves is shared memory reads: a 64 x 64 product took 10,400 cycles with 4 x 4
+// tiles, 4,096 being the pipe's bound.
 template <int BS>
-struct IluSmem {
-  static constexpr size_t BYTES = sizeof(double) * (2 * BS * BS + BS) + sizeof(int) * 2 * BS;
+struct BlkCfg {
+  static constexpr bool MMA = BS % 4 == 0 && BS > 4;
+  static constexpr int LD = MMA && BS % 16 != 4 ? (BS / 16 * 16 + 4 < BS ? BS / 16 * 16 + 20 : BS / 16 * 16 + 4) : BS;
+  static constexpr int NM = (BS + 7) / 8;                // 8-row tiles: warps of a product
+  static constexpr int KS = BS / 4;                      // its steps
+  static constexpr int NT4 = (BS + 3) / 4, TILES = NT4 * NT4;
+  static constexpr int WORK = MMA ? NM * 32 : TILES;     // threads of a product
+  static constexpr int ACC = MMA ? 2 * NM : 16;          // results per thread
+};
+static_assert(BlkCfg<64>::LD == 68 && BlkCfg<36>::LD == 36 && BlkCfg<16>::LD == 20 && BlkCfg<100>::LD == 100, "strides");
+
+// position (row, column) of a thread's n-th result
+template <int BS>
+__device__ inline int2 blk_pos(int n) {
+  using K = BlkCfg<BS>;
+  const int tid = threadIdx.x;
+  if constexpr (K::MMA) {
+    const int lane = tid & 31;
+    return make_int2((tid >> 5) * 8 + lane / 4, (n >> 1) * 8 + (lane % 4) * 2 + (n & 1));
+  } else {
+    return make_int2(tid / K::NT4 * 4 + n / 4, tid % K::NT4 * 4 + n % 4);
+  }
+}
+
+// acc = X Y; X and Y in shared memory with rows of LD doubles (whole warps call it)
+template <int BS>
+__device__ inline void blk_mul(const double* X, const double* Y, double (&acc)[BlkCfg<BS>::ACC]) {
+  using K = BlkCfg<BS>;
+  const int tid = threadIdx.x;
+  if constexpr (K::MMA) {
+    const int lane = tid & 31, w = tid >> 5;
+#pragma unroll
+    for (int n = 0; n < K::ACC; ++n) acc[n] = 0.0;
+    // rows and columns past the block meet clamped addresses; their results are not used
+    const int row = w * 8 + lane / 4;
+    const double* x = X + (row < BS ? row : BS - 1) * K::LD + lane % 4;
+    const double* y = Y + (lane % 4) * K::LD + lane / 4;
+    constexpr int LAST = (K::NM - 1) * 8;
+    const int yl = LAST + lane / 4 < BS ? LAST : LAST - (LAST + 8 - BS);
+#pragma unroll 4
+    for (int m = 0; m < K::KS; ++m) {
+      const double av = x[m * 4];
+#pragma unroll
+      for (int t = 0; t < K::NM; ++t) {
+        const double bv = y[m * 4 * K::LD + (t == K::NM - 1 ? yl : t * 8)];
+        asm("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0,%1}, {%2}, {%3}, {%0,%1};"
+            : "+d"(acc[2 * t]), "+d"(acc[2 * t + 1])
+            : "d"(av), "d"(bv));
+      }
+    }
+  } else {
+    double c[4][4];
+    block_gemm_tile<BS>(X, Y, tid / K::NT4 * 4, tid % K::NT4 * 4, c);
+#pragma unroll
+    for (int n = 0; n < 16; ++n) acc[n] = c[n / 4][n % 4];
+  }
+}
+
+// a thread's results to rows of ld doubles (global or shared); matrix form: pairs of columns
+template <int BS>
+__device__ inline void blk_store(const double (&acc)[BlkCfg<BS>::ACC], double* dst, int ld) {
+  using K = BlkCfg<BS>;
+  if constexpr (K::MMA) {
+#pragma unroll
+    for (int n = 0; n < K::ACC; n += 2) {
+      const int2 p = blk_pos<BS>(n);
+      if (p.x < BS && p.y < BS) *reinterpret_cast<double2*>(dst + p.x * ld + p.y) = make_double2(acc[n], acc[n + 1]);
+    }
+  } else {
+#pragma unroll
+    for (int n = 0; n < K::ACC; ++n) {
+      const int2 p = blk_pos<BS>(n);
+      if (p.x < BS && p.y < BS) dst[p.x * ld + p.y] = acc[n];
+    }
+  }
+}
+
+// copies a block to shared memory with rows of LD doubles (asynchronously)
+template <int BS>
+__device__ inline void block_fetch(double* dst, const double* __restrict__ src) {
+  constexpr int LD = BlkCfg<BS>::LD;
+  const unsigned d = (unsigned)__cvta_generic_to_shared(dst);
+  if constexpr (BS % 2 == 0) {
+    for (int t = threadIdx.x; t < BS * BS / 2; t += blockDim.x) {
+      const int o = LD == BS ? 2 * t : 2 * t / BS * LD + 2 * t % BS;
+      asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(d + o * 8), "l"(src + 2 * t) : "memory");
+    }
+  } else {
+    for (int t = threadIdx.x; t < BS * BS; t += blockDim.x)
+      asm volatile("cp.async.ca.shared.global [%0], [%1], 8;\n" ::"r"(d + t * 8), "l"(src + t) : "memory");
+  }
+}
+
+// One CTA factors one element's row. Both lower neighbours' operands are
+// requested at the start (cp.async) and the diagonal block stays in registers
+// through its updates and its inversion.
+//
+// Inversion: in-place Gauss-Jordan with partial pivoting. Rows are not exchanged:
+// the pivot of column k is the largest |a[i][k]| of the rows not yet used (first
+// index on ties), and with p_k that row the stored matrix S gives
+// inv[k][p_j] = S[p_k][j].
+//   matrix form (blk_invert): eight columns at a time. One warp takes the panel
+//     of those columns through its eight pivots alone (whole-warp maximum, no
+//     barrier, every lane forming its candidate's reciprocal meanwhile); with
+//     the panel M that leaves and the eight pivot rows R as they were, every
+//     other entry becomes a[i][j] (0 in a pivot row) + M[i] . R[:, j], two matrix
+//     instructions per 8 x 8 tile on the tiles the warps hold. Three barriers per
+//     eight pivots instead of a barrier and a selection among the warps for each.
+//   odd sizes (block_invert_regs): TPR threads per row, thread q holding columns
+//     q, q + TPR, ...; every warp offers its best row and all pick the winner.
+template <int BS>
+struct FacCfg {
+  using B = BlkCfg<BS>;
+  static constexpr int TPR = BS > 64 ? 4 : 2;
+  static constexpr int NC = (BS + TPR - 1) / TPR;        // columns per thread
+  static constexpr int NCP = (NC + 3) / 4 * 4 + 2;       // stride of a thread's part of an offer (16-byte reads of
+                                                         // the TPR parts fall in different banks)
+  static constexpr int GJ = BS * TPR;                    // threads of the inversion
+  static constexpr int GW = (GJ + 31) / 32;              // its warps
+  static constexpr int THREADS = ((B::WORK > GJ ? B::WORK : GJ) + 31) / 32 * 32;
+  static constexpr int B2 = BS * BS;
+  static constexpr int B2P = (BS * B::LD + 1) / 2 * 2;   // a staged block
+  // operand buffers: A_ek, inv(U_kk), A_ke of two neighbours, or (largest blocks) two buffers used in turn
+  static constexpr int NBUF = 6 * B2P * 8 <= 212 * 1024 ? 6 : 2;
+  static constexpr int OFFER = GW * TPR * NCP;           // doubles of one pivot's offers
+  // scratch of the inversion: the panel and the pivot rows, or the offers and candidates; pivot rows by column,
+  // columns by pivot row, flag
+  static constexpr int PS = 12, WK = B::MMA ? BS * PS + 8 * B::LD : 2 * OFFER + 4 * GW;
+  static constexpr size_t SMEM = sizeof(double) * ((size_t)NBUF * B2P + WK) + sizeof(int) * (2 * BS + 4);
+  static_assert(SMEM <= 227 * 1024, "the row's operands exceed the shared memory of one CTA");
 };
 
+// dst (global) = inverse of the block in shared memory at `a` (rows of LD), which is overwritten; false (uniform
+// over the CTA) if it is singular, dst then the identity
 template <int BS>
-__global__ void __launch_bounds__(256) ilu_level_kernel(int E, int nnzb, const int* __restrict__ elems,
-                                                        const int* __restrict__ rowptr,
-                                                        const int* __restrict__ colidx, double* __restrict__ LU,
-                                                        double* __restrict__ Uinv, int* flag) {
-  extern __shared__ double sh[];
-  double* X = sh;                  // BS x BS
-  double* Y = X + BS * BS;         // BS x BS
-  double* fcol = Y + BS * BS;      // BS
-  int* perm = reinterpret_cast<int*>(fcol + BS);
-  int* colsrc = perm + BS;
-  __shared__ int singular;
+__device__ inline bool block_invert_regs(double* a, double* offers, uint4* cand, int* perm, double* dst) {
+  using K = FacCfg<BS>;
+  constexpr int TPR = K::TPR, NC = K::NC, NCP = K::NCP, LD = BlkCfg<BS>::LD;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  bool singular = false;
+  double m[NC];
+  const bool mine = tid < K::GJ;
+  const int r = mine ? tid / TPR : 0, q = tid % TPR;
+  int kr = 0;  // the column whose pivot this row is
+  if (warp < K::GW) {
+#pragma unroll
+    for (int j = 0; j < NC; ++j) m[j] = mine && q + TPR * j < BS ? a[r * LD + q + TPR * j] : 0.0;
+    bool used = !mine;
+#pragma unroll
+    for (int j = 0; j < NC; ++j) {
+#pragma unroll
+      for (int qq = 0; qq < TPR; ++qq) {
+        const int k = qq + TPR * j;
+        if (k >= BS || singular) break;
+        const int par = k & 1;
+        double* offer = offers + par * K::OFFER;
+        const double f = __shfl_sync(0xffffffffu, m[j], (lane & ~(TPR - 1)) | qq);  // a[r][k]
+        // the warp's largest |a[i][k]| of the rows not used (a NaN counts as zero)
+        unsigned hi = 0, lo = 0;
+        if (!used && f == f) {
+          hi = (unsigned)__double2hiint(f) & 0x7fffffffu;
+          lo = (unsigned)__double2loint(f);
+        }
+        const unsigned mh = __reduce_max_sync(0xffffffffu, hi);
+        const unsigned ml = __reduce_max_sync(0xffffffffu, hi == mh ? lo : 0u);
+        const unsigned who = __ballot_sync(0xffffffffu, !used && hi == mh && lo == ml);
+        const int first = who ? __ffs(who) - 1 : 0;
+        if (who && lane / TPR == first / TPR) {
+          double2* o = reinterpret_cast<double2*>(offer + (warp * TPR + q) * NCP);
+#pragma unroll
+          for (int h = 0; h < (NC + 1) / 2; ++h) o[h] = make_double2(m[2 * h], 2 * h + 1 < NC ? m[2 * h + 1] : 0.0);
+        }
+        unsigned bh = mh, bl = ml, row = (unsigned)(warp * 32 + first) / TPR;
+        int bw = warp;
+        if constexpr (K::GW == 1) {
+          __syncwarp();
+        } else {
+          if (lane == 0) cand[par * K::GW + warp] = make_uint4(mh, ml, row, 0u);
+          asm volatile("bar.sync 1, %0;" ::"n"(K::GW * 32) : "memory");
+          // the winner: largest, then lowest warp (rows ascend with the warps)
+          bh = bl = 0;
+#pragma unroll
+          for (int w = 0; w < K::GW; ++w) {
+            const uint4 cw = cand[par * K::GW + w];
+            if (cw.x > bh || (cw.x == bh && cw.y > bl)) {
+              bh = cw.x;
+              bl = cw.y;
+              row = cw.z;
+              bw = w;
+            }
+          }
+        }
+        if ((bh | bl) == 0) {  // no nonzero pivot: uniform over the inversion's warps
+          singular = true;
+        } else {
+          if (tid == 0) perm[k] = (int)row;
+          const double* o = offer + bw * TPR * NCP;
+          const double ri = 1.0 / o[qq * NCP + j];
+          const double2* oq = reinterpret_cast<const double2*>(o + q * NCP);
+          const bool own = mine && r == (int)row;
+          // the pivot row becomes ri times itself, the others lose f ri times it: with z = 0 for the pivot row,
+          // both are z a[i] + g a[p]
+          const double g = own ? ri : -(f * ri);
+#pragma unroll
+          for (int h = 0; h < (NC + 1) / 2; ++h) {
+            const double2 pr = oq[h];
+#pragma unroll
+            for (int w = 0; w < 2; ++w)
+              if (2 * h + w < NC) m[2 * h + w] = fma(g, w ? pr.y : pr.x, own ? 0.0 : m[2 * h + w]);
+          }
+          if (q == qq) m[j] = g;
+          if (own) {
+            used = true;
+            kr = k;
+          }
+          if constexpr (K::GW == 1) __syncwarp();
+        }
+      }
+    }
+    if (tid == 0) perm[BS] = singular ? 1 : 0;
+  }
+  __syncthreads();
+  singular = perm[BS] != 0;
+  if (mine && !singular) {
+#pragma unroll
+    for (int j = 0; j < NC; ++j)
+      if (q + TPR * j < BS) a[kr * LD + perm[q + TPR * j]] = m[j];
+  }
+  __syncthreads();
+  for (int t = tid; t < BS * BS; t += blockDim.x) dst[t] = singular ? (t / BS == t % BS ? 1.0 : 0.0) : a[t / BS * LD + t % BS];
+  return !singular;
+}
+
+// the inverse of the block whose tiles the warps hold (C, as blk_mul's results) into dst (global), through out
+// (shared, rows of LD); work: the inversion's shared scratch; false (uniform over the CTA) if it is singular, dst
+// then the identity
+template <int BS>
+__device__ inline bool blk_invert(double (&C)[BlkCfg<BS>::ACC], double* out, double* work, int* perm, double* dst) {
+  using K = FacCfg<BS>;
+  using B = BlkCfg<BS>;
+  constexpr int LD = B::LD, NM = B::NM, PS = K::PS, RPL = (BS + 31) / 32;
+  double* PB = work;             // [BS][PS]: the panel
+  double* R = work + BS * PS;    // [8][LD]: its pivot rows before the update
+  int* rank = perm + BS;         // the column a row was pivot of (-1: not yet)
+  int* fail = rank + BS;
+  const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
+  const int row = w * 8 + lane / 4, q = lane % 4;
+  const bool mine = w < NM && row < BS;
+  for (int i = tid; i < BS; i += blockDim.x) rank[i] = -1;
+  if (tid == 0) *fail = 0;
+#pragma unroll
+  for (int t = 0; t < NM; ++t) {
+    constexpr int LASTC = BS - (NM - 1) * 8;
+    const int nc = t == NM - 1 ? LASTC : 8;  // columns of the panel (4 or 8)
+    if (mine && 2 * q < nc) *reinterpret_cast<double2*>(PB + row * PS + 2 * q) = make_double2(C[2 * t], C[2 * t + 1]);
+    __syncthreads();
+    if (w == 0) {
+      // the panel's pivots: lane l holds rows l, l + 32, ...
+      double p[RPL][8];
+      bool used[RPL];
+#pragma unroll
+      for (int rr = 0; rr < RPL; ++rr) {
+        const int r = lane + 32 * rr;
+        used[rr] = r >= BS || rank[r] >= 0;
+#pragma unroll
+        for (int c = 0; c < 8; ++c) p[rr][c] = r < BS && c < nc ? PB[r * PS + c] : 0.0;
+      }
+      bool bad = false;
+#pragma unroll
+      for (int c = 0; c < 8; ++c) {
+        if (c >= nc || bad) break;
+        // the lane's largest candidate (a NaN counts as zero; first row on ties) and its reciprocal
+        unsigned long long key = 0;
+        int br = 0;
+#pragma unroll
+        for (int rr = 0; rr < RPL; ++rr) {
+          const unsigned long long v = !used[rr] && p[rr][c] == p[rr][c]
+                                           ? (unsigned long long)__double_as_longlong(p[rr][c]) & 0x7fffffffffffffffull
+                                           : 0ull;
+          if (v > key) {
+            key = v;
+            br = rr;
+          }
+        }
+        double bv = p[0][c];
+#pragma unroll
+        for (int rr = 1; rr < RPL; ++rr) bv = br == rr ? p[rr][c] : bv;
+        const double rl = 1.0 / bv;
+        const unsigned hi = (unsigned)(key >> 32), lo = (unsigned)key;
+        const unsigned mh = __reduce_max_sync(0xffffffffu, hi);
+        const unsigned ml = __reduce_max_sync(0xffffffffu, hi == mh ? lo : 0u);
+        // the lowest row among equal candidates
+        const unsigned mr = __reduce_min_sync(0xffffffffu, hi == mh && lo == ml ? (unsigned)(lane + 32 * br) : ~0u);
+        if ((mh | ml) == 0) {
+          bad = true;
+          break;
+        }
+        const int src = mr & 31, sr = mr >> 5;  // uniform
+        const double ri = __shfl_sync(0xffffffffu, rl, src);
+        double pr[8];
+#pragma unroll
+        for (int k = 0; k < 8; ++k) {
+          double v = p[0][k];
+#pragma unroll
+          for (int rr = 1; rr < RPL; ++rr) v = sr == rr ? p[rr][k] : v;
+          pr[k] = __shfl_sync(0xffffffffu, v, src);
+        }
+#pragma unroll
+        for (int rr = 0; rr < RPL; ++rr) {
+          const bool own = lane == src && rr == sr;
+          const double g = own ? ri : -(p[rr][c] * ri);
+#pragma unroll
+          for (int k = 0; k < 8; ++k)
+            if (k != c) p[rr][k] = fma(g, pr[k], own ? 0.0 : p[rr][k]);
+          p[rr][c] = g;
+          used[rr] = used[rr] || own;
+        }
+        if (lane == 0) {
+          perm[t * 8 + c] = (int)mr;
+          rank[mr] = t * 8 + c;
+        }
+      }
+      if (bad) {
+        if (lane == 0) *fail = 1;
+      } else {
+#pragma unroll
+        for (int rr = 0; rr < RPL; ++rr) {
+          const int r = lane + 32 * rr;
+          if (r < BS) {
+#pragma unroll
+            for (int c = 0; c < 8; ++c)
+              if (c < nc) PB[r * PS + c] = p[rr][c];
+          }
+        }
+      }
+    }
+    __syncthreads();
+    if (*fail) break;  // uniform
+    // the pivot rows as they were, then out of the tiles
+    if (mine) {
+      const int k = rank[row] - t * 8;
+      if (k >= 0) {
+#pragma unroll
+        for (int n = 0; n < NM; ++n) {
+          if (n * 8 + 2 * q < BS) *reinterpret_cast<double2*>(R + k * LD + n * 8 + 2 * q) = make_double2(C[2 * n], C[2 * n + 1]);
+          C[2 * n] = C[2 * n + 1] = 0.0;
+        }
+      }
+    }
+    __syncthreads();
+    if (w < NM) {
+      const double* a = PB + (row < BS ? row : BS - 1) * PS + q;
+      const double a0 = a[0], a1 = nc > 4 ? a[4] : 0.0;
+      const double* b = R + q * LD + lane / 4;
+      constexpr int LAST = (NM - 1) * 8;
+      const int yl = LAST + lane / 4 < BS ? LAST : LAST - (LAST + 8 - BS);
+#pragma unroll
+      for (int n = 0; n < NM; ++n) {
+        if (n == t) continue;
+        const int o = n == NM - 1 ? yl : n * 8;
+        asm("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0,%1}, {%2}, {%3}, {%0,%1};"
+            : "+d"(C[2 * n]), "+d"(C[2 * n + 1])
+            : "d"(a0), "d"(b[o]));
+        if (nc > 4)
+          asm("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0,%1}, {%2}, {%3}, {%0,%1};"
+              : "+d"(C[2 * n]), "+d"(C[2 * n + 1])
+              : "d"(a1), "d"(b[4 * LD + o]));
+      }
+      const double2 v = mine && 2 * q < nc ? *reinterpret_cast<const double2*>(PB + row * PS + 2 * q) : make_double2(0.0, 0.0);
+      C[2 * t] = v.x;
+      C[2 * t + 1] = v.y;
+    }
+    __syncthreads();  // the panel and the pivot rows are read before the next ones are written
+  }
+  const bool singular = *fail != 0;
+  if (mine && !singular) {
+#pragma unroll
+    for (int n = 0; n < B::ACC; ++n) {
+      const int col = (n >> 1) * 8 + 2 * q + (n & 1);
+      if (col < BS) out[rank[row] * LD + perm[col]] = C[n];
+    }
+  }
+  __syncthreads();
+  for (int t = tid; t < BS * BS; t += blockDim.x) dst[t] = singular ? (t / BS == t % BS ? 1.0 : 0.0) : out[t / BS * LD + t % BS];
+  return !singular;
+}
+
+// What bounds it: the chain of BS pivots and the four block products of an inner
+// element. Whole factorisation and one apply, before (4 x 4 tiles, three barriers
+// per pivot with the block in shared memory) and now: Navier-Stokes 64 x 64 p = 2
+// 9.4 and 3.7 ms, p = 3 26.2 and 8.0 ms, 40 x 40 p = 4 50.4 and 17.4 ms; tiles of
+// 8, 128 x 128 p = 2 4.9 and 2.1 ms; Burgers 64 x 64 p = 2 2.9 and 1.9 ms.
+template <int BS>
+__global__ void __launch_bounds__(FacCfg<BS>::THREADS) ilu_level_kernel(int E, int nnzb, const int* __restrict__ elems,
+                                                                        const int* __restrict__ rowptr,
+                                                                        const int* __restrict__ colidx,
+                                                                        double* LU, double* Uinv, int* flag) {
+  using K = FacCfg<BS>;
+  using B = BlkCfg<BS>;
+  constexpr int B2 = K::B2, LD = B::LD;
+  extern __shared__ __align__(16) double sh[];
+  double* offers = sh + (size_t)K::NBUF * K::B2P;
+  int* perm = reinterpret_cast<int*>(offers + K::WK);
+  const int tid = threadIdx.x;
   const int e = elems[blockIdx.x];
   // block and element indices are checked before use: a bad one sets
   // *flag = 2 and the CTA leaves (the values are uniform over the CTA)
   if (e < 0 || e >= E || rowptr[e] < 0 || rowptr[e + 1] > nnzb) {
-    if (threadIdx.x == 0) atomicExch(flag, 2);
+    if (tid == 0) atomicExch(flag, 2);
     return;
   }
-  for (int kl = rowptr[e]; kl < rowptr[e + 1]; ++kl) {
-    const int k = colidx[kl];
-    if (k < 0 || k >= E) {
-      if (threadIdx.x == 0) atomicExch(flag, 2);
-      return;
+  const int b0 = rowptr[e];
+  const int kd = find_block(rowptr, colidx, e, e);
+  bool bad = kd < 0;
+  for (int kl = b0; !bad && kl < kd; ++kl) bad = colidx[kl] < 0 || colidx[kl] >= e;  // columns ascend
+  if (bad) {
+    if (tid == 0) atomicExch(flag, 2);
+    return;
+  }
+  // neighbour n's operands in buffers 3 n .. 3 n + 2 (A_ek, inv(U_kk), A_ke)
+  const int nl = kd - b0;
+  auto fetch = [&](int n) {
+    const int k = colidx[b0 + n];
+    double* buf = sh + (size_t)(K::NBUF == 6 ? 3 * (n & 1) : 0) * K::B2P;
+    block_fetch<BS>(buf, LU + (size_t)(b0 + n) * B2);
+    block_fetch<BS>(buf + K::B2P, Uinv + (size_t)k * B2);
+    if (K::NBUF == 6) {
+      const int ke = find_block(rowptr, colidx, k, e);
+      if (ke >= 0) block_fetch<BS>(buf + 2 * K::B2P, LU + (size_t)ke * B2);
     }
-    if (k >= e) break;  // columns ascend: the lower blocks come first
-    double* Aek = LU + (size_t)kl * BS * BS;
-    const double* Ui = Uinv + (size_t)k * BS * BS;
+    cp_async_commit();
+  };
+  if (nl > 0) fetch(0);
+  if (K::NBUF == 6 && nl > 1) fetch(1);
+  const bool work = tid < B::WORK;
+  double D[B::ACC], acc[B::ACC];
+#pragma unroll
+  for (int n = 0; n < B::ACC; ++n) {
+    const int2 p = blk_pos<BS>(n);
+    D[n] = work && p.x < BS && p.y < BS ? LU[(size_t)kd * B2 + p.x * BS + p.y] : 0.0;
+  }
+  for (int n = 0; n < nl; ++n) {
+    const int kl = b0 + n, k = colidx[kl];
+    double* X = sh + (size_t)(K::NBUF == 6 ? 3 * (n & 1) : 0) * K::B2P;
+    double* Y = X + K::B2P;
+    if (K::NBUF == 6 && n + 1 < nl) cp_async_wait<1>();
+    else cp_async_wait<0>();
     __syncthreads();
-    for (int t = threadIdx.x; t < BS * BS; t += blockDim.x) {
-      X[t] = Aek[t];
-      Y[t] = Ui[t];
+    // L_ek = A_ek inv(U_kk) over A_ek (matrix form: a warp reads and writes its own rows only)
+    if (work) blk_mul<BS>(X, Y, acc);
+    if (B::MMA) __syncwarp();
+    else __syncthreads();
+    if (work) {
+      blk_store<BS>(acc, X, LD);
+      blk_store<BS>(acc, LU + (size_t)kl * B2, BS);
     }
-    __syncthreads();
-    // L_ek = A_ek inv(U_kk): kept in registers until every thread has read X
-    constexpr int NT = (BS + 3) / 4;
-    constexpr int MAXT = (NT * NT + 255) / 256;
-    double keep[MAXT][4][4];
-    int slot = 0;
-    block_gemm<BS>(X, Y, [&](int r0, int c0, double (&acc)[4][4]) {
-#pragma unroll
-      for (int a = 0; a < 4; ++a)
-#pragma unroll
-        for (int b = 0; b < 4; ++b) keep[slot][a][b] = acc[a][b];
-      ++slot;
-    });
-    __syncthreads();
-    slot = 0;
-    for (int tt = threadIdx.x; tt < NT * NT; tt += blockDim.x, ++slot) {
-      const int r0 = (tt / NT) * 4, c0 = (tt % NT) * 4;
-#pragma unroll
-      for (int a = 0; a < 4; ++a)
-#pragma unroll
-        for (int b = 0; b < 4; ++b)
-          if (r0 + a < BS && c0 + b < BS) {
-            X[(r0 + a) * BS + c0 + b] = keep[slot][a][b];
-            Aek[(r0 + a) * BS + c0 + b] = keep[slot][a][b];
-          }
-    }
-    // A_ej -= L_ek U_kj for the upper blocks of row k that lie in row e's pattern
+    if (B::MMA) __syncwarp();
+    else __syncthreads();
+    // A_ej -= L_ek U_kj for the upper blocks of row k that lie in row e's pattern (on a quadrilateral grid: e's
+    // own diagonal block only)
+    bool have_z = K::NBUF == 6;  // A_ke is in its buffer
     for (int kj = rowptr[k]; kj < rowptr[k + 1]; ++kj) {
       const int jc = colidx[kj];
       if (jc <= k) continue;
-      const int ej = find_block(rowptr, colidx, e, jc);
+      const int ej = jc == e ? kd : find_block(rowptr, colidx, e, jc);
       if (ej < 0) continue;  // outside the pattern: dropped (level 0 fill)
-      if (kj >= nnzb || ej >= nnzb) {
-        if (threadIdx.x == 0) atomicExch(flag, 2);
+      if (kj >= nnzb || ej >= nnzb) {  // uniform over the CTA
+        if (tid == 0) atomicExch(flag, 2);
+        cp_async_wait<0>();
         return;
       }
-      const double* Akj = LU + (size_t)kj * BS * BS;
-      double* Aej = LU + (size_t)ej * BS * BS;
-      __syncthreads();
-      for (int t = threadIdx.x; t < BS * BS; t += blockDim.x) Y[t] = Akj[t];
-      __syncthreads();
-      block_gemm<BS>(X, Y, [&](int r0, int c0, double (&acc)[4][4]) {
+      double* Z = K::NBUF == 6 ? X + 2 * K::B2P : Y;
+      if (!have_z || jc != e) {
+        have_z = false;
+        __syncthreads();
+        for (int t = tid; t < B2; t += blockDim.x) Z[t / BS * LD + t % BS] = LU[(size_t)kj * B2 + t];
+        __syncthreads();
+      }
+      if (work) {
+        blk_mul<BS>(X, Z, acc);
 #pragma unroll
-        for (int a = 0; a < 4; ++a)
-#pragma unroll
-          for (int b = 0; b < 4; ++b)
-            if (r0 + a < BS && c0 + b < BS) Aej[(r0 + a) * BS + c0 + b] -= acc[a][b];
-      });
+        for (int m = 0; m < B::ACC; ++m) {
+          const int2 p = blk_pos<BS>(m);
+          if (jc == e) D[m] -= acc[m];
+          else if (p.x < BS && p.y < BS) LU[(size_t)ej * B2 + p.x * BS + p.y] -= acc[m];
+        }
+      }
+    }
+    // buffers of this neighbour are free
+    if (n + (K::NBUF == 6 ? 2 : 1) < nl) {
+      __syncthreads();
+      fetch(n + (K::NBUF == 6 ? 2 : 1));
     }
   }
+  if (work && nl > 0) blk_store<BS>(D, LU + (size_t)kd * B2, BS);
   __syncthreads();
-  const int kd = find_block(rowptr, colidx, e, e);
-  if (kd < 0) {
-    if (threadIdx.x == 0) atomicExch(flag, 2);
-    return;
+  bool ok;
+  if constexpr (B::MMA) {
+    ok = blk_invert<BS>(D, sh, offers, perm, Uinv + (size_t)e * B2);
+  } else {
+    if (work) blk_store<BS>(D, sh, LD);
+    __syncthreads();
+    ok = block_invert_regs<BS>(sh, offers, reinterpret_cast<uint4*>(offers + 2 * K::OFFER), perm, Uinv + (size_t)e * B2);
   }
-  const double* Aee = LU + (size_t)kd * BS * BS;
-  for (int t = threadIdx.x; t < BS * BS; t += blockDim.x) X[t] = Aee[t];
-  __syncthreads();
-  gj_invert<BS>(X, perm, fcol, &singular);
-  __syncthreads();
-  if (singular && threadIdx.x == 0) atomicExch(flag, 1);
-  write_inverse<BS>(X, perm, colsrc, singular, Uinv + (size_t)e * BS * BS);
+  if (!ok && tid == 0) atomicExch(flag, 1);
 }
 
 // After the factorisation every upper block is scaled by the inverse of its
@@ -197,33 +599,42 @@ __global__ void __launch_bounds__(256) ilu_level_kernel(int E, int nnzb, const i
 // substitution y_e = inv(U_ee) (f_e - sum_{k>e} U_ek y_k) becomes
 //   y_e = inv(U_ee) f_e - sum_{k>e} (inv(U_ee) U_ek) y_k,
 // a plain block-row product whose rows can be split across warps.
-// One CTA per row, both operands staged in shared memory.
+// One CTA per row, the operands staged in shared memory.
 template <int BS>
-__global__ void __launch_bounds__(256) ilu_scale_upper_kernel(int E, const int* __restrict__ rowptr,
-                                                              const int* __restrict__ colidx,
-                                                              double* __restrict__ LU,
-                                                              const double* __restrict__ Uinv) {
-  extern __shared__ double sh[];
-  double* D = sh;            // BS x BS
-  double* B = sh + BS * BS;  // BS x BS
+struct ScaleCfg {
+  static constexpr int THREADS = (BlkCfg<BS>::WORK + 31) / 32 * 32;
+  static constexpr int B2P = FacCfg<BS>::B2P;
+  static constexpr size_t SMEM = sizeof(double) * 2 * B2P;
+};
+
+template <int BS>
+__global__ void __launch_bounds__(ScaleCfg<BS>::THREADS) ilu_scale_upper_kernel(int E, const int* __restrict__ rowptr,
+                                                                                const int* __restrict__ colidx,
+                                                                                double* LU,
+                                                                                const double* __restrict__ Uinv) {
+  using B = BlkCfg<BS>;
+  extern __shared__ __align__(16) double sh[];
+  double* D = sh;
+  double* U = sh + ScaleCfg<BS>::B2P;
   const int e = blockIdx.x;
   if (e >= E) return;
-  const double* Di = Uinv + (size_t)e * BS * BS;
-  for (int t = threadIdx.x; t < BS * BS; t += blockDim.x) D[t] = Di[t];
+  block_fetch<BS>(D, Uinv + (size_t)e * BS * BS);
   for (int kb = rowptr[e]; kb < rowptr[e + 1]; ++kb) {
     if (colidx[kb] <= e) continue;
-    double* U = LU + (size_t)kb * BS * BS;
+    double* g = LU + (size_t)kb * BS * BS;
     __syncthreads();
-    for (int t = threadIdx.x; t < BS * BS; t += blockDim.x) B[t] = U[t];
+    block_fetch<BS>(U, g);
+    cp_async_commit();
+    cp_async_wait<0>();
     __syncthreads();
-    block_gemm<BS>(D, B, [&](int r0, int c0, double (&acc)[4][4]) {
-#pragma unroll
-      for (int a = 0; a < 4; ++a)
-#pragma unroll
-        for (int b = 0; b < 4; ++b)
-          if (r0 + a < BS && c0 + b < BS) U[(r0 + a) * BS + c0 + b] = acc[a][b];
-    });
+    if (threadIdx.x < B::WORK) {
+      double acc[B::ACC];
+      blk_mul<BS>(D, U, acc);
+      blk_store<BS>(acc, g, BS);
+    }
   }
+  cp_async_commit();
+  cp_async_wait<0>();  // a row without upper blocks still has its first copy in flight
 }
 
 // ------------------------------------------------------------- reductions
@@ -476,16 +887,17 @@ cudaError_t la_ilu_factor(const DeviceMesh& dm, const int* order, const std::vec
   const int bs = dm.nb * dm.neq;
 #define ICX_ILUF_CASE(B)                                                                               \
   if (bs == B) {                                                                                       \
-    cudaError_t e = smem_attr(ilu_level_kernel<B>, IluSmem<B>::BYTES);                                 \
-    if (e == cudaSuccess) e = smem_attr(ilu_scale_upper_kernel<B>, IluSmem<B>::BYTES);                 \
+    cudaError_t e = smem_attr(ilu_level_kernel<B>, FacCfg<B>::SMEM);                                   \
+    if (e == cudaSuccess) e = smem_attr(ilu_scale_upper_kernel<B>, ScaleCfg<B>::SMEM);                 \
     if (e != cudaSuccess) return e;                                                                    \
     for (size_t l = 0; l + 1 < lvl_off.size(); ++l) {                                                  \
       const int cnt = lvl_off[l + 1] - lvl_off[l];                                                     \
       if (cnt > 0)                                                                                     \
-        ilu_level_kernel<B><<<cnt, 256, IluSmem<B>::BYTES, s>>>(dm.E, dm.nnzb, order + lvl_off[l],     \
-                                                                dm.bsr_rowptr, dm.bsr_colidx, LU, Uinv, flag); \
+        ilu_level_kernel<B><<<cnt, FacCfg<B>::THREADS, FacCfg<B>::SMEM, s>>>(                          \
+            dm.E, dm.nnzb, order + lvl_off[l], dm.bsr_rowptr, dm.bsr_colidx, LU, Uinv, flag);          \
     }                                                                                                  \
-    ilu_scale_upper_kernel<B><<<dm.E, 256, IluSmem<B>::BYTES, s>>>(dm.E, dm.bsr_rowptr, dm.bsr_colidx, LU, Uinv); \
+    ilu_scale_upper_kernel<B><<<dm.E, ScaleCfg<B>::THREADS, ScaleCfg<B>::SMEM, s>>>(                   \
+        dm.E, dm.bsr_rowptr, dm.bsr_colidx, LU, Uinv);                                                 \
     return cudaGetLastError();                                                                         \
   }
   ICX_BLOCK_SIZES(ICX_ILUF_CASE)
