@@ -64,6 +64,8 @@ struct StripArgs {
   int* err;
   int depth;   // chunks in the ring
   int cluster; // CTAs per cluster (1: every hand-over through the exchange rows)
+  int sweep;   // 0 both sweeps in one launch (all CTAs resident), 1 the forward one, 2 the backward one
+  unsigned long long* ticket;  // sweep 1 and 2: tickets drawn by the clusters so far
 };
 
 // completion barriers of the staged copies
@@ -431,10 +433,17 @@ __device__ inline bool strip_sweep(const StripArgs<TA>& a, int s, StripShared<BS
   return true;
 }
 
-// strips are dealt to the CTAs round-robin in order; every CTA runs its forward
-// sweeps in ascending, then its backward sweeps in descending order. A strip
-// waits only for the one before (after) it, and the whole grid is resident, so
-// the first unfinished strip can always run.
+// One launch for both sweeps: strips are dealt to the CTAs round-robin in order;
+// every CTA runs its forward sweeps in ascending, then its backward sweeps in
+// descending order. A strip waits only for the one before (after) it, and the
+// whole grid is resident (cooperative launch), so the first unfinished strip can
+// always run.
+// One launch per sweep: every CTA runs one strip, and the clusters draw tickets
+// as they start, ascending strips for the forward, descending ones for the
+// backward sweep. A strip then waits only for a CTA of its own cluster or for a
+// cluster that drew before it, so nothing needs to be resident: for plans larger
+// than the GPU, and for several applies side by side (cooperative launches run
+// one after the other).
 template <int BS, class TA>
 __global__ void __launch_bounds__((StripCfg<BS, TA>::NT)) ilu_apply_strip_kernel(StripArgs<TA> a) {
   using K = StripCfg<BS, TA>;
@@ -445,6 +454,16 @@ __global__ void __launch_bounds__((StripCfg<BS, TA>::NT)) ilu_apply_strip_kernel
   if (threadIdx.x < 2) sh.stop[threadIdx.x] = 0;
   if (threadIdx.x < K::DMAX) mbar_init((unsigned)__cvta_generic_to_shared(sh.bars + threadIdx.x), 1);
   asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  __shared__ unsigned drawn;
+  const int ncl = gridDim.x / a.cluster;
+  if (a.sweep && cluster_rank() == 0 && threadIdx.x == 0)
+    drawn = (unsigned)(atomicAdd(a.ticket, 1ull) % (unsigned long long)ncl);
+  if (a.sweep) {
+    cluster_sync();
+    unsigned t;
+    asm volatile("ld.shared::cluster.u32 %0, [%1];" : "=r"(t) : "r"(cluster_map((unsigned)__cvta_generic_to_shared(&drawn), 0)) : "memory");
+    s = (int)(a.sweep == 1 ? t : ncl - 1 - t) * a.cluster + (int)cluster_rank();
+  }
   if (a.cluster > 1) {
     const int n = s < a.nstrips ? a.strips[s].nx * BS : 0;
     for (int i = threadIdx.x; i < n; i += K::NT) inbox[i] = __longlong_as_double((long long)FLOW_SENTINEL);
@@ -454,8 +473,13 @@ __global__ void __launch_bounds__((StripCfg<BS, TA>::NT)) ilu_apply_strip_kernel
   }
   unsigned gch = 0;
   bool ok = true;
-  for (; ok && s < a.nstrips; s += gridDim.x) ok = strip_sweep<BS, TA, true>(a, s, sh, ring, inbox, gch);
-  for (s -= gridDim.x; ok && s >= 0; s -= gridDim.x) ok = strip_sweep<BS, TA, false>(a, s, sh, ring, inbox, gch);
+  if (a.sweep == 0) {
+    for (; ok && s < a.nstrips; s += gridDim.x) ok = strip_sweep<BS, TA, true>(a, s, sh, ring, inbox, gch);
+    for (s -= gridDim.x; ok && s >= 0; s -= gridDim.x) ok = strip_sweep<BS, TA, false>(a, s, sh, ring, inbox, gch);
+  } else if (s < a.nstrips) {
+    if (a.sweep == 1) strip_sweep<BS, TA, true>(a, s, sh, ring, inbox, gch);
+    else strip_sweep<BS, TA, false>(a, s, sh, ring, inbox, gch);
+  }
   // no CTA of a cluster ends while another may still store into its inbox
   if (a.cluster > 1) cluster_sync();
 }
@@ -503,7 +527,7 @@ __global__ void strip_fill_kernel(long long n, double* ex) {
 }
 
 template <int BS, class TA>
-cudaError_t launch_strips(const IluStripPlan& p, const StripArgs<TA>& args, cudaStream_t s) {
+cudaError_t launch_strips(const IluStripPlan& p, const StripArgs<TA>& args, bool side_by_side, cudaStream_t s) {
   using K = StripCfg<BS, TA>;
   constexpr auto kern = ilu_apply_strip_kernel<BS, TA>;
   constexpr int kSmem = 224 * 1024, kCluster = 8;
@@ -512,12 +536,12 @@ cudaError_t launch_strips(const IluStripPlan& p, const StripArgs<TA>& args, cuda
   if (e == cudaSuccess) e = cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
   if (e != cudaSuccess) return e;
   StripArgs<TA> a = args;
-  // clusters of strips that hand their rows over in shared memory, where the whole plan is resident that way
-  // (one strip per CTA) and the inbox (a row of the widest grid) leaves room for two chunks
+  // clusters of strips that hand their rows over in shared memory, where the inbox (a row of the widest grid)
+  // leaves room for two chunks; side by side with other applies no more than two, so that several CTAs share an SM
   const long long inbox = (long long)p.max_nx * BS * 8;
   const long long fit = (kSmem - K::VD * K::VB - inbox) / K::CHUNK;
-  if (p.nstrips > 1 && fit >= 2) {
-    a.depth = (int)std::min<long long>(4, fit);  // deeper rings gain nothing here and keep other sets off the SM
+  if (fit >= 2) {
+    a.depth = (int)std::min<long long>(side_by_side ? 2 : 4, fit);
     cudaLaunchConfig_t cfg = {};
     cfg.blockDim = dim3(K::NT);
     cfg.dynamicSmemBytes = (size_t)a.depth * K::CHUNK + K::VD * K::VB + inbox;
@@ -530,27 +554,30 @@ cudaError_t launch_strips(const IluStripPlan& p, const StripArgs<TA>& args, cuda
     cfg.attrs = attr;
     e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)cfg.dynamicSmemBytes);
     if (e != cudaSuccess) return e;
-    // the largest cluster whose grid is resident (clusters of 8 leave some SMs of a GPU cluster empty)
-    for (int cl = kCluster; cl > 1; cl /= 2) {
-      cfg.gridDim = dim3((p.nstrips + cl - 1) / cl * cl);
-      attr[0].val.clusterDim.x = cl;
-      cfg.numAttrs = 1;
-      int clusters = 0;
-      if (cudaOccupancyMaxActiveClusters(&clusters, kern, &cfg) != cudaSuccess) {
-        (void)cudaGetLastError();
-        continue;
-      }
-      if ((long long)clusters * cl < cfg.gridDim.x) continue;
+    cfg.gridDim = dim3((p.nstrips + kCluster - 1) / kCluster * kCluster);
+    attr[0].val.clusterDim.x = a.cluster = kCluster;
+    cfg.numAttrs = 1;
+    int clusters = 0;
+    if (cudaOccupancyMaxActiveClusters(&clusters, kern, &cfg) != cudaSuccess) {
+      (void)cudaGetLastError();
+      clusters = 0;
+    }
+    // one cooperative launch for both sweeps where the whole grid is resident (saves a launch and the tickets)
+    if (!side_by_side && (long long)clusters * kCluster >= cfg.gridDim.x) {
       cfg.numAttrs = 2;
-      a.cluster = cl;
+      a.sweep = 0;
       return cudaLaunchKernelEx(&cfg, kern, a);
     }
+    if (clusters > 0) {
+      for (a.sweep = 1; a.sweep <= 2; ++a.sweep)
+        if ((e = cudaLaunchKernelEx(&cfg, kern, a)) != cudaSuccess) return e;
+      return cudaSuccess;
+    }
   }
-  // every hand-over through L2: still ahead of the data-flow apply (256 x 256, 36 x 36 blocks, FP64: 1.47 ms
-  // against 1.70), but not for 36 x 36 blocks in FP32 (1.86 against 1.56)
-  if (BS >= 36 && sizeof(TA) == 4) return cudaErrorNotSupported;
+  // rows too wide for an inbox: every hand-over through L2
   a.depth = (int)std::min<long long>(K::DMAX, (kSmem - K::VD * K::VB) / K::CHUNK);
   a.cluster = 1;
+  a.sweep = 0;
   const size_t smem = (size_t)a.depth * K::CHUNK + K::VD * K::VB;
   int per_sm = 0;
   e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
@@ -573,11 +600,11 @@ cudaError_t pack_strips(const IluStripPlan& p, const double* LU, const double* U
 
 template <class TA>
 cudaError_t apply_strips(int bs, const IluStripPlan& p, const TA* pk, const double* x, double* y, double* f, int* err,
-                         cudaStream_t s) {
+                         bool side_by_side, cudaStream_t s) {
   if (p.nstrips < 1 || !pk) return cudaErrorInvalidValue;
-  StripArgs<TA> a{p.nstrips, p.strips, reinterpret_cast<const unsigned char*>(pk), x, f, y, p.ex, err, 0, 1};
+  StripArgs<TA> a{p.nstrips, p.strips, reinterpret_cast<const unsigned char*>(pk), x, f, y, p.ex, err, 0, 1, 0, p.ticket};
 #define ICX_STRIP_CASE(B) \
-  if (bs == B) return launch_strips<B, TA>(p, a, s);
+  if (bs == B) return launch_strips<B, TA>(p, a, side_by_side, s);
   ICX_STRIP_SIZES(ICX_STRIP_CASE)
 #undef ICX_STRIP_CASE
   return cudaErrorNotSupported;
@@ -621,12 +648,12 @@ cudaError_t la_ilu_strip_pack_f32(int bs, const IluStripPlan& p, const double* L
   return pack_all<float>(bs, p, LU, Uinv, pk, s);
 }
 cudaError_t la_ilu_apply_strips(int bs, const IluStripPlan& p, const double* pk, const double* x, double* y, double* f,
-                                int* err, cudaStream_t s) {
-  return apply_strips<double>(bs, p, pk, x, y, f, err, s);
+                                int* err, bool side_by_side, cudaStream_t s) {
+  return apply_strips<double>(bs, p, pk, x, y, f, err, side_by_side, s);
 }
 cudaError_t la_ilu_apply_strips_f32(int bs, const IluStripPlan& p, const float* pk, const double* x, double* y,
-                                    double* f, int* err, cudaStream_t s) {
-  return apply_strips<float>(bs, p, pk, x, y, f, err, s);
+                                    double* f, int* err, bool side_by_side, cudaStream_t s) {
+  return apply_strips<float>(bs, p, pk, x, y, f, err, side_by_side, s);
 }
 
 }  // namespace icx

@@ -65,6 +65,7 @@ struct IluStripPlan {
   double* ex = nullptr;        // [nex], shared by both precisions' plans
   long long nex = 0;
   long long bytes = 0;         // packed factors
+  unsigned long long* ticket = nullptr;  // [1], shared by both precisions' plans: clusters started so far
 };
 // rows per strip for a block size (0: no strip kernel for it)
 constexpr int ilu_strip_rows(int bs) { return bs <= 4 ? 8 : bs <= 9 ? 4 : bs <= 16 ? 4 : bs <= 25 ? 2 : bs <= 36 ? 1 : 0; }
@@ -76,11 +77,12 @@ cudaError_t la_ilu_strip_pack(int bs, const IluStripPlan& p, const double* LU, c
                               cudaStream_t s);
 cudaError_t la_ilu_strip_pack_f32(int bs, const IluStripPlan& p, const double* LU, const double* Uinv, float* pk,
                                   cudaStream_t s);
-// y = (LU)^-1 x; f = n doubles of scratch; *err = 1 if a wait ran out
+// y = (LU)^-1 x; f = n doubles of scratch; *err = 1 if a wait ran out; side_by_side: applies of other plans run
+// at the same time on other streams
 cudaError_t la_ilu_apply_strips(int bs, const IluStripPlan& p, const double* pk, const double* x, double* y, double* f,
-                                int* err, cudaStream_t s);
+                                int* err, bool side_by_side, cudaStream_t s);
 cudaError_t la_ilu_apply_strips_f32(int bs, const IluStripPlan& p, const float* pk, const double* x, double* y,
-                                    double* f, int* err, cudaStream_t s);
+                                    double* f, int* err, bool side_by_side, cudaStream_t s);
 cudaError_t la_block_diag_correct_f32(int E, int bs, const float* D, const double* y, double* z, cudaStream_t s);
 // *d_out = x . y (device scalar, overwritten)
 cudaError_t la_dot_to(long long n, const double* x, const double* y, double* d_out, cudaStream_t s);

@@ -184,6 +184,9 @@ struct icx_pset {
   double* h_hcol = nullptr;           // pinned copy of hcol
   double* h_small = nullptr;          // pinned [n_parts][m + 2] staging
   cudaStream_t cap = nullptr;         // graph capture stream
+  std::vector<cudaStream_t> side;     // all_groups: a stream per group but the last, its completion, the fork
+  std::vector<cudaEvent_t> joined;
+  cudaEvent_t forked = nullptr;
   std::vector<cudaGraphExec_t> exec;  // Arnoldi step graphs (step j)
   std::vector<int> seen;
   unsigned long long key = 0;
@@ -270,12 +273,40 @@ cudaError_t put_per_part(icx_pset* S, const std::vector<double>& v, double* dst,
   return cudaMemcpyAsync(dst, S->h_small, sizeof(double) * S->n_parts * lda, cudaMemcpyHostToDevice, s);
 }
 
-cudaError_t all_groups(icx_pset* S, const std::function<cudaError_t(icx_ctx*, long long)>& f) {
-  for (size_t g = 0; g < S->groups.size(); ++g) {
-    cudaError_t e = f(S->groups[g], S->group_off[g]);
-    if (e != cudaSuccess) return e;
+// f for every group, the groups side by side: the last (the highest order, the
+// longest) on stream q, the others on side streams that start after q's work so
+// far and that q then waits for. The groups' buffers are their own and their
+// parts of the set's vectors do not overlap; their launches are bound by latency
+// (the block-ILU(0) apply above all) and leave most of the GPU to one another:
+// set of 16 problems, orders 1 to 4, PSET_MEASURED. Works the same
+// under stream capture (the fork and the join become edges of the graph).
+cudaError_t all_groups(icx_pset* S, cudaStream_t q,
+                       const std::function<cudaError_t(icx_ctx*, long long, cudaStream_t)>& f) {
+  const size_t n = S->groups.size();
+  cudaError_t e = cudaSuccess;
+  while (e == cudaSuccess && S->side.size() + 1 < n) {
+    cudaStream_t t = nullptr;
+    cudaEvent_t ev = nullptr;
+    if ((e = cudaStreamCreateWithFlags(&t, cudaStreamNonBlocking)) != cudaSuccess) break;
+    S->side.push_back(t);
+    if ((e = cudaEventCreateWithFlags(&ev, cudaEventDisableTiming)) == cudaSuccess) S->joined.push_back(ev);
   }
-  return cudaSuccess;
+  if (e == cudaSuccess && n > 1 && !S->forked) e = cudaEventCreateWithFlags(&S->forked, cudaEventDisableTiming);
+  if (e == cudaSuccess && n > 1) e = cudaEventRecord(S->forked, q);
+  size_t begun = 0;
+  for (size_t g = 0; g + 1 < n && e == cudaSuccess; ++g) {
+    if ((e = cudaStreamWaitEvent(S->side[g], S->forked, 0)) != cudaSuccess) break;
+    ++begun;
+    e = f(S->groups[g], S->group_off[g], S->side[g]);
+  }
+  if (e == cudaSuccess && n > 0) e = f(S->groups[n - 1], S->group_off[n - 1], q);
+  // every stream begun is joined, also after an error
+  for (size_t g = 0; g < begun; ++g) {
+    cudaError_t j = cudaEventRecord(S->joined[g], S->side[g]);
+    if (j == cudaSuccess) j = cudaStreamWaitEvent(q, S->joined[g], 0);
+    if (e == cudaSuccess) e = j;
+  }
+  return e;
 }
 
 struct Kry {
@@ -349,9 +380,9 @@ icx_status pset_gmres(icx_pset* S, int pc, bool mixed, int m, int maxit, double 
       double* vj = S->V + (size_t)j * N;
       double* vj1 = S->V + (size_t)(j + 1) * N;
       auto step = [&](cudaStream_t q) -> cudaError_t {
-        cudaError_t e = all_groups(S, [&](icx_ctx* g, long long off) -> cudaError_t {
-          cudaError_t ee = pc ? icx::solver_apply_pc(g, pc, mixed, vj + off, S->z + off, q) : cudaSuccess;
-          if (ee == cudaSuccess) ee = icx::solver_operator(g, mixed, (pc ? S->z : vj) + off, vj1 + off, q);
+        cudaError_t e = all_groups(S, q, [&](icx_ctx* g, long long off, cudaStream_t t) -> cudaError_t {
+          cudaError_t ee = pc ? icx::solver_apply_pc(g, pc, mixed, vj + off, S->z + off, t) : cudaSuccess;
+          if (ee == cudaSuccess) ee = icx::solver_operator(g, mixed, (pc ? S->z : vj) + off, vj1 + off, t);
           return ee;
         });
         for (int pass = 0; pass < passes && e == cudaSuccess; ++pass) {
@@ -454,14 +485,16 @@ icx_status pset_gmres(icx_pset* S, int pc, bool mixed, int m, int maxit, double 
       PCK(cudaGetLastError());
     }
     if (pc) {
-      PCK(all_groups(S, [&](icx_ctx* g, long long off) {
-        return icx::solver_apply_pc(g, pc, mixed, S->w + off, S->z + off, s);
+      PCK(all_groups(S, s, [&](icx_ctx* g, long long off, cudaStream_t t) {
+        return icx::solver_apply_pc(g, pc, mixed, S->w + off, S->z + off, t);
       }));
       PCK(icx::la_axpby(N, 1.0, S->z, 1.0, x, s));
     } else {
       PCK(icx::la_axpby(N, 1.0, S->w, 1.0, x, s));
     }
-    PCK(all_groups(S, [&](icx_ctx* g, long long off) { return icx::solver_operator(g, mixed, x + off, S->w + off, s); }));
+    PCK(all_groups(S, s, [&](icx_ctx* g, long long off, cudaStream_t t) {
+      return icx::solver_operator(g, mixed, x + off, S->w + off, t);
+    }));
     PCK(icx::la_xpay(N, b, -1.0, S->w, S->r, s));
     std::vector<double> beta;
     rs = seg_norms(S, S->r, beta, s);
@@ -572,6 +605,9 @@ void icx_pset_destroy(icx_pset* S) {
   cudaSetDevice(S->device);
   free_buffers(S);
   if (S->cap) cudaStreamDestroy(S->cap);
+  for (cudaStream_t t : S->side) cudaStreamDestroy(t);
+  for (cudaEvent_t ev : S->joined) cudaEventDestroy(ev);
+  if (S->forked) cudaEventDestroy(S->forked);
   void* dev[] = {S->d_cbeg, S->d_cend, S->d_cpart, S->d_pck};
   for (void* p : dev)
     if (p) cudaFree(p);
@@ -591,8 +627,8 @@ icx_status icx_pset_residual(icx_pset* S, const double* d_u, double* d_res) {
   if (!S || !d_u || !d_res) return ICX_ERR_INVALID;
   cudaSetDevice(S->device);
   cudaStream_t s = 0;
-  PCK(all_groups(S, [&](icx_ctx* g, long long off) {
-    return icx::launch_residual(g->dm, g->phys, d_u + off, d_res + off, s);
+  PCK(all_groups(S, s, [&](icx_ctx* g, long long off, cudaStream_t t) {
+    return icx::launch_residual(g->dm, g->phys, d_u + off, d_res + off, t);
   }));
   PCK(cudaStreamSynchronize(s));
   return ICX_OK;
@@ -614,7 +650,8 @@ icx_status icx_pset_newton_solve(icx_pset* S, double* d_u, const icx_newton_opti
   icx_status st = ensure_buffers(S, m);
   if (st != ICX_OK) return st;
   for (icx_ctx* g : S->groups) {
-    st = icx::solver_group_ready(g, opt->precision, opt->pc_sweeps, opt->ilu_tile, opt->cuda_graphs != 0);
+    st = icx::solver_group_ready(g, opt->precision, opt->pc_sweeps, opt->ilu_tile, opt->cuda_graphs != 0,
+                                 S->groups.size() > 1);
     if (st != ICX_OK) return perr(S, st, std::string("group solver buffers: ") + g->err);
   }
   icx_pset_stats local_stats{};
@@ -624,8 +661,8 @@ icx_status icx_pset_newton_solve(icx_pset* S, double* d_u, const icx_newton_opti
   std::vector<icx_newton_report> R(P);
   for (auto& r : R) std::memset(&r, 0, sizeof(r));
   auto linearise = [&]() -> cudaError_t {
-    return all_groups(S, [&](icx_ctx* g, long long off) {
-      return icx::solver_linearise(g, d_u + off, S->res + off, opt->precision, s);
+    return all_groups(S, s, [&](icx_ctx* g, long long off, cudaStream_t t) {
+      return icx::solver_linearise(g, d_u + off, S->res + off, opt->precision, t);
     });
   };
   PCK(linearise());
@@ -649,7 +686,7 @@ icx_status icx_pset_newton_solve(icx_pset* S, double* d_u, const icx_newton_opti
     for (int p = 0; p < P; ++p) any = any || active[p];
     if (!any) break;
     ++stt.newton_rounds;
-    PCK(all_groups(S, [&](icx_ctx* g, long long) { return icx::solver_build_pc(g, pc, mixed, s); }));
+    PCK(all_groups(S, s, [&](icx_ctx* g, long long, cudaStream_t t) { return icx::solver_build_pc(g, pc, mixed, t); }));
     for (icx_ctx* g : S->groups) {
       int fl = 0;
       PCK(cudaMemcpyAsync(&fl, icx::solver_flag(g), sizeof(int), cudaMemcpyDeviceToHost, s));
@@ -699,8 +736,8 @@ icx_status icx_pset_newton_solve(icx_pset* S, double* d_u, const icx_newton_opti
         seg_xpay_kernel<<<S->n_chunks, kThreads, 0, s>>>(S->d_cbeg, S->d_cend, S->d_cpart, d_u, S->coef, S->du,
                                                         S->ut);
         PCK(cudaGetLastError());
-        PCK(all_groups(S, [&](icx_ctx* g, long long off) {
-          return icx::launch_residual(g->dm, g->phys, S->ut + off, S->rt + off, s);
+        PCK(all_groups(S, s, [&](icx_ctx* g, long long off, cudaStream_t t) {
+          return icx::launch_residual(g->dm, g->phys, S->ut + off, S->rt + off, t);
         }));
         std::vector<double> phi;
         st = seg_norms(S, S->rt, phi, s);

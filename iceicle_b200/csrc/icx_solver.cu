@@ -102,6 +102,7 @@ struct icx_solver_work {
   icx::IluStripPlan sp[2];
   void* spk[2] = {nullptr, nullptr};
   bool sp_ok[2] = {false, false};
+  bool side_by_side = false;  // the context is a group of a set, whose applies run at the same time
   IluTilePlan tp;           // tiled block-ILU(0) pattern and schedule (tp.tile == c->ilu_tile once built)
   int* pc_err = nullptr;    // set by the ILU apply if a dependency wait timed out
   double* dh = nullptr;     // device scalars (dot results)
@@ -250,6 +251,9 @@ icx_status build_strip_plan(icx_ctx* c) {
   double* ex = nullptr;
   CK(cudaMalloc((void**)&ex, sizeof(double) * nex));
   w->sp[0].ex = w->sp[1].ex = ex;
+  CK(cudaMalloc((void**)&w->sp[0].ticket, sizeof(unsigned long long)));
+  CK(cudaMemset(w->sp[0].ticket, 0, sizeof(unsigned long long)));
+  w->sp[1].ticket = w->sp[0].ticket;
   for (int pi = 0; pi < 2; ++pi) {
     icx::IluStripPlan& sp = w->sp[pi];
     sp.nex = nex;
@@ -515,8 +519,10 @@ cudaError_t ilu_flow(icx_ctx* c, bool mixed, const double* x, double* z, cudaStr
   // shape of the data-flow apply, same results, replaces it where it is faster)
   if (w->sp_ok[pi] && strip_shape(c, mixed)) {
     const cudaError_t e =
-        mixed ? icx::la_ilu_apply_strips_f32(w->bs, w->sp[1], (const float*)w->spk[1], x, z, w->pct, w->pc_err, s)
-              : icx::la_ilu_apply_strips(w->bs, w->sp[0], (const double*)w->spk[0], x, z, w->pct, w->pc_err, s);
+        mixed ? icx::la_ilu_apply_strips_f32(w->bs, w->sp[1], (const float*)w->spk[1], x, z, w->pct, w->pc_err,
+                                             w->side_by_side, s)
+              : icx::la_ilu_apply_strips(w->bs, w->sp[0], (const double*)w->spk[0], x, z, w->pct, w->pc_err,
+                                         w->side_by_side, s);
     if (e != cudaErrorNotSupported) return e;  // not ahead at this size: the data-flow apply, same results
   }
   if (!sen && rows != w->flow_rows) {
@@ -814,7 +820,7 @@ void free_solver_work(icx_ctx* c) {
   icx_solver_work* w = c->sw;
   void* ptrs[] = {w->pc16, w->uinv16, w->V32, w->vt, w->vals32, w->pc32, w->uinv32, w->vals, w->pc, w->uinv, w->V, w->w, w->z, w->r, w->res, w->du,
                   w->ustep, w->rwork, w->pct, w->pct2, w->pct3, w->pct4, w->order, w->cnt, w->cnt_rows, w->pc_err,
-                  w->dh, w->flag, w->lw.partial, w->sp[0].strips, w->sp[1].strips, w->sp[0].ex, w->spk[0], w->spk[1]};
+                  w->dh, w->flag, w->lw.partial, w->sp[0].strips, w->sp[1].strips, w->sp[0].ex, w->sp[0].ticket, w->spk[0], w->spk[1]};
   w->graphs.release();
   for (void* p : ptrs)
     if (p) cudaFree(p);
@@ -1302,13 +1308,14 @@ cudaError_t solver_apply_ilu_flow(icx_ctx* c, bool mixed, const double* x, doubl
 }
 
 // ---- the pieces a batch of independent solves drives per group context
-icx_status solver_group_ready(icx_ctx* c, int precision, int pc_sweeps, int ilu_tile, bool graphs) {
+icx_status solver_group_ready(icx_ctx* c, int precision, int pc_sweeps, int ilu_tile, bool graphs, bool side_by_side) {
   // one Krylov vector of the group's own: the batch holds the Krylov basis
   icx_status st = ensure_work(c, 1);
   if (st != ICX_OK) return st;
   if (precision >= 1 && (st = ensure_mixed(c)) != ICX_OK) return st;
   c->sw->sweeps = pc_sweeps;
   c->sw->graphs_on = graphs;
+  c->sw->side_by_side = side_by_side;
   if (ilu_tile >= 0) c->ilu_tile = ilu_tile;
   return ICX_OK;
 }
