@@ -382,7 +382,10 @@ __device__ inline void node_perturbed(const int* fixmask, const double* fixval, 
   }
 }
 
-// Jacobian work items, one thread each; item = {type, k_or_t, obj, aux, slot, side}
+// Jacobian work items, one thread each; item = {type, k_or_t, obj, aux, slot, side}, grouped by
+// type.  Bound by the latency of one thread's two evaluations (244 registers, 8 warps an SM), so a
+// warp that holds several types pays for each of them in turn: 148 us in the order of the nodes,
+// 65 us grouped (64 x 64 elements, P1, all interior nodes free).
 //   type 0: dICE/du   trace t (obj), perturbed DOF aux of side `side`
 //   type 1: dR/dx     node k, element obj (volume integral), component aux
 //   type 2: dR/dx     node k, face obj (trace / boundary integral), component aux
@@ -889,6 +892,16 @@ icx_status build_mdg_pattern(icx_ctx* c) {
     }
   }
   m.nitems = (int)items.size() / 6;
+  // grouped by type, each group in the order above (the slots stay where they are): a warp of
+  // mdg_jac_kernel then runs one of its four bodies instead of up to three in turn
+  {
+    std::vector<int> by;
+    by.reserve(items.size());
+    for (int type = 0; type < 4; ++type)
+      for (size_t i = 0; i < items.size(); i += 6)
+        if (items[i] == type) by.insert(by.end(), items.begin() + i, items.begin() + i + 6);
+    items.swap(by);
+  }
   m.nslots = slot;
   // entries: (row, col, source)
   long long nbsr = (long long)dm.nnzb * bs * bs;
