@@ -25,6 +25,7 @@
 #include <algorithm>
 #include <vector>
 
+#include "icx_bulk.cuh"
 #include "icx_internal.h"
 #include "icx_linalg.h"
 #include "icx_blockrow.cuh"
@@ -67,32 +68,6 @@ struct StripArgs {
   int sweep;   // 0 both sweeps in one launch (all CTAs resident), 1 the forward one, 2 the backward one
   unsigned long long* ticket;  // sweep 1 and 2: tickets drawn by the clusters so far
 };
-
-// completion barriers of the staged copies
-__device__ inline void mbar_init(unsigned bar, unsigned count) {
-  asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(bar), "r"(count) : "memory");
-}
-__device__ inline void mbar_expect(unsigned bar, unsigned bytes) {
-  asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
-}
-// waits for the phase; bounded like the other waits (a copy in flight always lands)
-__device__ inline bool mbar_wait(unsigned bar, unsigned parity) {
-  for (unsigned spins = 0; spins < ICX_FLOW_SPINS; ++spins) {
-    unsigned ok;
-    asm volatile(
-        "{\n.reg .pred p;\nmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\nselp.u32 %0, 1, 0, p;\n}\n"
-        : "=r"(ok)
-        : "r"(bar), "r"(parity)
-        : "memory");
-    if (ok) return true;
-  }
-  return false;
-}
-__device__ inline void bulk_copy(unsigned dst, const void* src, unsigned bytes, unsigned bar) {
-  asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(dst),
-               "l"(src), "r"(bytes), "r"(bar)
-               : "memory");
-}
 
 // a row handed over inside a cluster goes straight into the consumer's shared memory
 __device__ inline unsigned cluster_rank() {

@@ -145,6 +145,19 @@ cudaError_t la_ilu_apply_groups_bf16(const DeviceMesh& dm, const IluGroupShape& 
                                      const int* glev, const int* glev_ptr, int ctas, const __nv_bfloat16* LU,
                                      const __nv_bfloat16* Uinv, const double* x, double* y, double* f, int* err,
                                      cudaStream_t s);
+// the group apply with the factors streamed through shared memory
+// (icx_ilu_tile.cu; FP64: the data-flow apply's sums); cudaErrorNotSupported:
+// block bytes no multiple of 16, or the group's vectors and three elements do
+// not fit
+cudaError_t la_ilu_apply_tiles(const DeviceMesh& dm, const IluGroupShape& gs, const int* task, const int* glev,
+                               const int* glev_ptr, const double* LU, const double* Uinv, const double* x,
+                               double* y, int* err, cudaStream_t s);
+cudaError_t la_ilu_apply_tiles(const DeviceMesh& dm, const IluGroupShape& gs, const int* task, const int* glev,
+                               const int* glev_ptr, const float* LU, const float* Uinv, const double* x,
+                               double* y, int* err, cudaStream_t s);
+cudaError_t la_ilu_apply_tiles(const DeviceMesh& dm, const IluGroupShape& gs, const int* task, const int* glev,
+                               const int* glev_ptr, const __nv_bfloat16* LU, const __nv_bfloat16* Uinv,
+                               const double* x, double* y, int* err, cudaStream_t s);
 bool group_rows_bf16_fits(const DeviceMesh& dm, const IluGroupShape& gs);
 // y = x rounded to BF16
 cudaError_t la_d2bf(long long n, const double* x, __nv_bfloat16* y, cudaStream_t s);

@@ -498,11 +498,23 @@ cudaError_t ilu_flow(icx_ctx* c, bool mixed, const double* x, double* z, cudaStr
     const IluTilePlan& tp = w->tp;
     const icx::IluGroupShape gs{tp.ngroups, tp.gmax, tp.nlev_max, gsched, tp.gloc};
     const int ctas = dm.tile.flow_ctas[pi];
+    // the factors streamed through shared memory, where they fit: at the
+    // default shape in FP64 (the tuned ones are the other group applies, same
+    // results), at every schedule-5 shape in FP32 and BF16
+    const bool bf16 = mixed && w->bf16 && w->pc16;
+    cudaError_t e = cudaErrorNotSupported;
+    if (bf16)
+      e = icx::la_ilu_apply_tiles(dm, gs, tp.gtask, tp.glev, tp.glev_ptr, w->pc16, w->uinv16, x, z, w->pc_err, s);
+    else if (mixed && gsched == 5)
+      e = icx::la_ilu_apply_tiles(dm, gs, tp.gtask, tp.glev, tp.glev_ptr, w->pc32, w->uinv32, x, z, w->pc_err, s);
+    else if (!mixed && gsched == 4 && (ctas == 0 || ctas == 2) && rows == icx::flow_rows_default(w->bs))
+      e = icx::la_ilu_apply_tiles(dm, gs, tp.gtask, tp.glev, tp.glev_ptr, w->pc, w->uinv, x, z, w->pc_err, s);
+    if (e != cudaErrorNotSupported) return e;
     // BF16 factors: the one-lane-per-row form where it fits, else the FP32
     // copies. Its CTA size follows the group size (measured at 256 x 256,
     // p = 2: 8 x 8 tiles 0.159 ms with 128 threads against 0.191 with 256;
     // 16 x 16 tiles 0.240 ms with 256 against 0.322 with 128)
-    if (mixed && w->bf16 && w->pc16 && icx::group_rows_bf16_fits(dm, gs)) {
+    if (bf16 && icx::group_rows_bf16_fits(dm, gs)) {
       const int ctas16 = tp.gmax <= 64 ? 3 : tp.gmax <= 256 ? 2 : 1;
       return icx::la_ilu_apply_groups_bf16(dm, gs, tp.gtask, tp.glev, tp.glev_ptr, ctas16, w->pc16, w->uinv16, x,
                                            z, w->pct, w->pc_err, s);
