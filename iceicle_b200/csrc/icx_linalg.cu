@@ -643,12 +643,15 @@ __global__ void __launch_bounds__(ScaleCfg<BS>::THREADS) ilu_scale_upper_kernel(
 // over x: each thread holds x_i once per group of G basis vectors, so x is
 // read ceil(nvec / G) times instead of nvec times (the vectors V_j once
 // each); per block the sums are reduced by shuffles, then across the warps in
-// a fixed order
+// a fixed order. With a ticket the last block to finish adds the blocks'
+// partial sums as mdot_final_kernel does, in the same order: for small grids
+// and few vectors that is over before a second launch would have begun
 template <class TV, int G>
 __global__ void __launch_bounds__(256) mdot_grouped_kernel(long long n, const TV* __restrict__ V, long long ld,
-                                                           int nvec, const double* __restrict__ x,
-                                                           double* __restrict__ partial) {
+                                                           int nvec, const double* __restrict__ x, double* partial,
+                                                           unsigned* ticket, double* __restrict__ out) {
   __shared__ double red[G][8];
+  __shared__ bool last;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   for (int j0 = 0; j0 < nvec; j0 += G) {
     double acc[G];
@@ -673,8 +676,33 @@ __global__ void __launch_bounds__(256) mdot_grouped_kernel(long long n, const TV
 #pragma unroll
       for (int w = 0; w < 8; ++w) s += red[threadIdx.x][w];
       partial[(size_t)(j0 + threadIdx.x) * gridDim.x + blockIdx.x] = s;
+      if (ticket) __threadfence();
     }
     __syncthreads();
+  }
+  if (!ticket) return;
+  // the counter wraps to 0 with the last block: ready for the next launch
+  if (threadIdx.x == 0) last = atomicInc(ticket, gridDim.x - 1) == gridDim.x - 1;
+  __syncthreads();
+  if (!last) return;
+  __threadfence();
+  for (int j = warp; j < nvec; j += 8) {
+    double v[8];  // what threads lane, lane + 32, ... of mdot_final_kernel hold
+#pragma unroll
+    for (int k = 0; k < 8; ++k) v[k] = 0.0;
+    for (int b0 = 0; b0 < (int)gridDim.x; b0 += 256)
+#pragma unroll
+      for (int k = 0; k < 8; ++k) {
+        const int b = b0 + lane + 32 * k;
+        if (b < (int)gridDim.x) v[k] += __ldcg(partial + (size_t)j * gridDim.x + b);
+      }
+#pragma unroll
+    for (int h = 4; h > 0; h >>= 1)
+#pragma unroll
+      for (int k = 0; k < h; ++k) v[k] += v[k + h];
+#pragma unroll
+    for (int off = 16; off > 0; off >>= 1) v[0] += __shfl_down_sync(0xffffffffu, v[0], off);
+    if (lane == 0) out[j] = v[0];
   }
 }
 
@@ -749,20 +777,35 @@ static int grid_for(long long n) {
   return (int)(g < 148 * 8 ? (g < 1 ? 1 : g) : 148 * 8);
 }
 
+// a block per 256 rows up to kMdotBlocks (blocks without a row would add zeros). Up to a block per SM the last one
+// sums the partials: a Krylov step of 9216 unknowns 98 us against 107; with 1184 blocks their fences and tickets
+// cost more than the second launch (a norm of 589824 values 11.0 us against 6.4 + 2.3)
+template <class TV>
+static cudaError_t mdot(LinalgWork& w, long long n, const TV* V, long long ld, int nvec, const double* x,
+                        double* d_out, cudaStream_t s) {
+  const int nb = grid_for(n);
+  static_assert(kMdotBlocks == 148 * 8, "grid_for's bound");
+  const bool fuse = nb <= kMdotFuse;
+  mdot_grouped_kernel<TV, 8><<<nb, 256, 0, s>>>(n, V, ld, nvec, x, w.partial, fuse ? w.ticket() : nullptr, d_out);
+  if (!fuse) mdot_final_kernel<<<nvec, 256, 0, s>>>(nb, nvec, w.partial, d_out);
+  return cudaGetLastError();
+}
+
 cudaError_t la_mdot(LinalgWork& w, long long n, const double* V, long long ld, int nvec, const double* x,
                     double* d_out, cudaStream_t s) {
-  const int nb = kMdotBlocks;
-  mdot_grouped_kernel<double, 8><<<nb, 256, 0, s>>>(n, V, ld, nvec, x, w.partial);
-  mdot_final_kernel<<<nvec, 256, 0, s>>>(nb, nvec, w.partial, d_out);
-  return cudaGetLastError();
+  return mdot(w, n, V, ld, nvec, x, d_out, s);
 }
 
 cudaError_t la_mdot32(LinalgWork& w, long long n, const float* V, long long ld, int nvec, const double* x,
                       double* d_out, cudaStream_t s) {
-  const int nb = kMdotBlocks;
-  mdot_grouped_kernel<float, 8><<<nb, 256, 0, s>>>(n, V, ld, nvec, x, w.partial);
-  mdot_final_kernel<<<nvec, 256, 0, s>>>(nb, nvec, w.partial, d_out);
-  return cudaGetLastError();
+  return mdot(w, n, V, ld, nvec, x, d_out, s);
+}
+
+cudaError_t la_mdot_alloc(LinalgWork& w) {
+  if (w.partial) return cudaSuccess;
+  cudaError_t e = cudaMalloc((void**)&w.partial, sizeof(double) * (64 * kMdotBlocks + 1));
+  if (e == cudaSuccess) e = cudaMemset(w.ticket(), 0, sizeof(double));
+  return e;
 }
 
 cudaError_t la_maxpy(long long n, const double* V, long long ld, int nvec, const double* d_h, double sign, double* w,

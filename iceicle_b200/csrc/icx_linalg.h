@@ -12,10 +12,13 @@ namespace icx {
 // CTAs of the multi-dot's first stage (8 per SM: enough warps in flight to
 // stream the basis at full bandwidth)
 constexpr int kMdotBlocks = 148 * 8;
+constexpr int kMdotFuse = 148;  // blocks up to which the dot products' last one adds the partial sums itself
 
 struct LinalgWork {
-  double* partial = nullptr;  // [64 vectors][kMdotBlocks] partial dot products
+  double* partial = nullptr;  // [64 vectors][kMdotBlocks] partial dot products, then the ticket
+  unsigned* ticket() const { return reinterpret_cast<unsigned*>(partial + 64 * kMdotBlocks); }
 };
+cudaError_t la_mdot_alloc(LinalgWork& w);
 
 // d_out[j] = V_j . x for j < nvec, V_j = V + j * ld (deterministic two-stage reduction)
 cudaError_t la_mdot(LinalgWork& w, long long n, const double* V, long long ld, int nvec, const double* x,
