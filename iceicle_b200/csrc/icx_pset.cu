@@ -42,6 +42,12 @@ constexpr long long kChunk = 4096;  // unknowns per reduction chunk (a chunk lie
 constexpr int kThreads = 256;
 constexpr int kPer = (int)(kChunk / kThreads);
 
+// Blocks side by side on one chunk (blockIdx.y): a set's unknowns make some 100 chunks, fewer than
+// there are SMs, so the vectors of a dot product and the rows of an update are spread over them. The
+// sums keep their order. A step of 30 vectors over 16 problems of 64 to 4096 elements: update
+// 62 -> 24 us, dot products 22 -> 13 us.
+constexpr int kSplit = 8;
+
 // partial[c * ldp + j] = sum over chunk c of V_j . x   (V_j = V + j * ld)
 __global__ void __launch_bounds__(kThreads) seg_dot_partial_kernel(const long long* __restrict__ cbeg,
                                                                    const long long* __restrict__ cend,
@@ -57,7 +63,7 @@ __global__ void __launch_bounds__(kThreads) seg_dot_partial_kernel(const long lo
     xv[t] = k < e ? x[k] : 0.0;
   }
   __shared__ double red[kThreads / 32];
-  for (int j = 0; j < nvec; ++j) {
+  for (int j = blockIdx.y; j < nvec; j += gridDim.y) {
     const double* v = V + (size_t)j * ld;
     double s = 0.0;
 #pragma unroll
@@ -98,8 +104,9 @@ __global__ void seg_maxpy_kernel(const long long* __restrict__ cbeg, const long 
                                  const double* __restrict__ coef, int ldc, double sign, double* __restrict__ w) {
   const int c = blockIdx.x;
   const double* h = coef + (size_t)cpart[c] * ldc;
-  for (long long k = cbeg[c] + threadIdx.x; k < cend[c]; k += blockDim.x) {
+  for (long long k = cbeg[c] + blockIdx.y * blockDim.x + threadIdx.x; k < cend[c]; k += gridDim.y * blockDim.x) {
     double s = 0.0;
+#pragma unroll 8
     for (int j = 0; j < nvec; ++j) s += h[j] * V[(size_t)j * ld + k];
     w[k] += sign * s;
   }
@@ -251,7 +258,7 @@ icx_status ensure_buffers(icx_pset* S, int m) {
 cudaError_t seg_dots(icx_pset* S, const double* V, long long ld, int nvec, const double* x, double* out, int ldo,
                      cudaStream_t s) {
   const int ldp = S->m + 2;
-  seg_dot_partial_kernel<<<S->n_chunks, kThreads, 0, s>>>(S->d_cbeg, S->d_cend, V, ld, nvec, x, S->partial, ldp);
+  seg_dot_partial_kernel<<<dim3(S->n_chunks, std::min(nvec, kSplit)), kThreads, 0, s>>>(S->d_cbeg, S->d_cend, V, ld, nvec, x, S->partial, ldp);
   seg_dot_final_kernel<<<(S->n_parts + 7) / 8, 256, 0, s>>>(S->n_parts, S->d_pck, S->partial, ldp, nvec, out, ldo);
   return cudaGetLastError();
 }
@@ -389,8 +396,8 @@ icx_status pset_gmres(icx_pset* S, int pc, bool mixed, int m, int maxit, double 
           double* slot = S->dots + (size_t)pass * P * ld;
           e = seg_dots(S, S->V, N, j + 1, vj1, slot, ld, q);
           if (e == cudaSuccess) {
-            seg_maxpy_kernel<<<S->n_chunks, kThreads, 0, q>>>(S->d_cbeg, S->d_cend, S->d_cpart, S->V, N, j + 1, slot, ld,
-                                                             -1.0, vj1);
+            seg_maxpy_kernel<<<dim3(S->n_chunks, kSplit), kThreads, 0, q>>>(S->d_cbeg, S->d_cend, S->d_cpart, S->V, N,
+                                                                            j + 1, slot, ld, -1.0, vj1);
             e = cudaGetLastError();
           }
         }
@@ -480,7 +487,7 @@ icx_status pset_gmres(icx_pset* S, int pc, bool mixed, int m, int maxit, double 
     PCK(cudaMemcpyAsync(S->coef, S->h_small, sizeof(double) * P * ld, cudaMemcpyHostToDevice, s));
     PCK(cudaMemsetAsync(S->w, 0, sizeof(double) * N, s));
     if (jmax > 0) {
-      seg_maxpy_kernel<<<S->n_chunks, kThreads, 0, s>>>(S->d_cbeg, S->d_cend, S->d_cpart, S->V, N, jmax, S->coef, ld,
+      seg_maxpy_kernel<<<dim3(S->n_chunks, kSplit), kThreads, 0, s>>>(S->d_cbeg, S->d_cend, S->d_cpart, S->V, N, jmax, S->coef, ld,
                                                        1.0, S->w);
       PCK(cudaGetLastError());
     }
