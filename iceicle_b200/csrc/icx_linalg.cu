@@ -646,7 +646,7 @@ __global__ void __launch_bounds__(ScaleCfg<BS>::THREADS) ilu_scale_upper_kernel(
 // a fixed order. Few rows per thread make that reduction the larger part, so a
 // warp folds its G sums together (9 exchanges for 8 sums instead of 40, the
 // same values) and a single vector takes G = 1: 15 FP32 vectors of 589824
-// values 19.9 -> 18.3 us, a norm 6.4 -> 3.7 us. With a ticket the last block to finish adds the blocks'
+// values 19.9 -> 18.3 us, a norm 6.4 -> 3.7 us (both with 1184 blocks). With a ticket the last block to finish adds the blocks'
 // partial sums as mdot_final_kernel does, in the same order: for small grids
 // and few vectors that is over before a second launch would have begun
 template <class TV, int G>
@@ -660,6 +660,7 @@ __global__ void __launch_bounds__(256) mdot_grouped_kernel(long long n, const TV
     double acc[G];
 #pragma unroll
     for (int g = 0; g < G; ++g) acc[g] = 0.0;
+#pragma unroll 2
     for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
       const double xi = x[i];
 #pragma unroll
@@ -781,8 +782,7 @@ static int grid_for(long long n) {
 template <class TV>
 static cudaError_t mdot(LinalgWork& w, long long n, const TV* V, long long ld, int nvec, const double* x,
                         double* d_out, cudaStream_t s) {
-  const int nb = grid_for(n);
-  static_assert(kMdotBlocks == 148 * 8, "grid_for's bound");
+  const int nb = std::min(grid_for(n), kMdotBlocks);
   const bool fuse = nb <= kMdotFuse;
   unsigned* ticket = fuse ? w.ticket() : nullptr;
   if (nvec == 1) mdot_grouped_kernel<TV, 1><<<nb, 256, 0, s>>>(n, V, ld, nvec, x, w.partial, ticket, d_out);

@@ -9,9 +9,11 @@
 
 namespace icx {
 
-// CTAs of the multi-dot's first stage (8 per SM: enough warps in flight to
-// stream the basis at full bandwidth)
-constexpr int kMdotBlocks = 148 * 8;
+// most CTAs of the multi-dot's first stage: 4 per SM, all that its registers
+// leave resident (of 8 the second half waited for the first: a norm of 589824
+// values 3.7 + 3.1 us against 3.0 + 2.3, 15 FP32 vectors 18.3 + 3.1 against
+// 20.3 + 2.3; a 128 x 128 Newton solve with BF16 tiles 413 ms against 401)
+constexpr int kMdotBlocks = 148 * 4;
 constexpr int kMdotFuse = 148;  // blocks up to which the dot products' last one adds the partial sums itself
 
 struct LinalgWork {
