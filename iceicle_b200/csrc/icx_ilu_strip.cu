@@ -22,6 +22,10 @@
 // sums are taken in the order of the data-flow apply (32 column accumulators
 // added pairwise at distances 16, 8, 4, 2, 1), so the results are the same bit
 // for bit.
+//
+// Against the data-flow apply, whose every level is a trip through L2 (FP64 /
+// FP32): NS p = 2 256 x 256 1.70 -> 1.02 / 1.56 -> 0.91 ms, 128 x 128 715 -> 452
+// us; a Newton solve on 32 x 32 Burgers elements (P2) 131 -> 71 ms.
 #include <algorithm>
 #include <vector>
 

@@ -13,8 +13,9 @@
 // the group share one vector in shared memory (an element's forward result is
 // read by its own warp alone before the backward result takes its place).
 //
-// The sums are those of the data-flow apply, value for value: 32 partial sums
-// over the columns modulo 32, folded at distance 16, 8, 4, 2, 1 (warp_row_sums).
+// The sums (the row kernel's apart) are those of the data-flow apply, value for
+// value: 32 partial sums over the columns modulo 32, folded at distance 16, 8,
+// 4, 2, 1 (warp_row_sums).
 // A lane holds the partial sums (k LPR + g) VEC + i, so distances down to
 // LPR VEC fold inside the lane, the next ones across the row's lanes, the last
 // ones inside the lane again.
@@ -133,7 +134,8 @@ struct TileLane {
 
 // the row's sum, on each of its lanes
 template <int BS, class TS>
-__device__ inline typename ComputeOf<TS>::type tile_row_sum(typename ComputeOf<TS>::type (&acc)[TileCfg<BS, TS>::KN][TileCfg<BS, TS>::VEC]) {
+__device__ inline typename ComputeOf<TS>::type tile_row_sum(
+    typename ComputeOf<TS>::type (&acc)[TileCfg<BS, TS>::KN][TileCfg<BS, TS>::VEC]) {
   using K = TileCfg<BS, TS>;
 #pragma unroll
   for (int h = K::KN / 2; h >= 1; h /= 2)
@@ -192,7 +194,8 @@ struct TileShared {
 
 // table and barriers of the group; false (uniform over the CTA): a plan out of its bounds
 template <int BS, class TS>
-__device__ inline bool tile_setup(const IluGroupArgs<TS>& a, int nslot, TileShared& sh, unsigned char* dsm, TileCta<TS>& c) {
+__device__ inline bool tile_setup(const IluGroupArgs<TS>& a, int nslot, TileShared& sh, unsigned char* dsm,
+                                  TileCta<TS>& c) {
   using K = TileCfg<BS, TS>;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int gid = blockIdx.x, gm = a.plan.gmax;
@@ -229,7 +232,8 @@ __device__ inline bool tile_setup(const IluGroupArgs<TS>& a, int nslot, TileShar
   for (int i = warp; i < G; i += blockDim.x / 32) {
     const int e = a.plan.task[pg0 + i].x;
     if (e >= 0 && e < a.E)
-      for (int k = lane * 16; k < BS; k += 512) asm volatile("prefetch.global.L2 [%0];" ::"l"(a.x + (size_t)e * BS + k));
+      for (int k = lane * 16; k < BS; k += 512)
+        asm volatile("prefetch.global.L2 [%0];" ::"l"(a.x + (size_t)e * BS + k));
   }
   if (threadIdx.x < nslot) {
     sh.held[threadIdx.x] = -1;
@@ -254,7 +258,8 @@ __device__ inline void tile_produce(const IluGroupArgs<TS>& a, int nslot, TileSh
     if (more) {
       if (n < nslot || mbar_test(c.empty + 8 * lane, phase)) {
         const int4 t = c.tab[n];
-        const unsigned bar = c.full + 8 * lane, dst = (unsigned)__cvta_generic_to_shared(c.ring + (size_t)lane * K::SLOT);
+        const unsigned bar = c.full + 8 * lane;
+        const unsigned dst = (unsigned)__cvta_generic_to_shared(c.ring + (size_t)lane * K::SLOT);
         const bool dg = t.x >= 0 && n >= c.G;
         const unsigned nb = t.x >= 0 ? ((t.w & 0xffff ? 1 : 0) + (t.w >> 16 ? 1 : 0)) * K::BB : 0;
         *(volatile int*)(sh.held + lane) = n;
@@ -420,7 +425,8 @@ __device__ inline void tile_row_madd(const TS* arow, const float* xs, float (&ac
 }
 
 template <int BS, class TS>
-__global__ void __launch_bounds__(TileRowCfg<BS>::NT + 32, 2) ilu_apply_tile_rows_kernel(IluGroupArgs<TS> a, int nslot) {
+__global__ void __launch_bounds__(TileRowCfg<BS>::NT + 32, 2)
+    ilu_apply_tile_rows_kernel(IluGroupArgs<TS> a, int nslot) {
   using K = TileCfg<BS, TS>;
   using R = TileRowCfg<BS>;
   extern __shared__ __align__(128) unsigned char dsm[];
@@ -501,7 +507,8 @@ __global__ void __launch_bounds__(TileRowCfg<BS>::NT + 32, 2) ilu_apply_tile_row
     // the chunk's rows are done, also those of the other warps: its slots go back, its results are there to read
     {
       int all = ok;
-      asm volatile("{\n.reg .pred p, q;\nsetp.ne.s32 p, %0, 0;\nbarrier.cta.red.and.pred q, 1, %1, p;\nselp.s32 %0, 1, 0, q;\n}"
+      asm volatile("{\n.reg .pred p, q;\nsetp.ne.s32 p, %0, 0;\nbarrier.cta.red.and.pred q, 1, %1, p;\n"
+                   "selp.s32 %0, 1, 0, q;\n}"
                    : "+r"(all)
                    : "n"(R::NT)
                    : "memory");
@@ -534,7 +541,9 @@ cudaError_t tile_launch(const IluGroupArgs<TS>& args, int nlev_max, cudaStream_t
   const int sms = device_attr(cudaDevAttrMultiProcessorCount);
   if (optin <= 0 || sms <= 0) return cudaErrorNotSupported;
   // as many CTAs on an SM as there are groups for (FP32 up to three, the row kernel two; FP64 reaches the copy
-  // rate with one) while each keeps a ring worth having
+  // rate with one) while each keeps a ring worth having: four slots, the row kernel eight, since a chunk takes
+  // that many at once (16 x 16 tiles in BF16: 212 us with one CTA of 16 slots, 272 with two of 4). Eight consumer
+  // warps where the CTA has the SM to itself, four where three share it (FP32, 128 x 128: 71 us against 77)
   const int gmax = args.plan.gmax, most = sizeof(TS) == 8 ? 1 : tile_by_rows<BS, TS>() ? 2 : 3;
   const int want = std::min(most, (args.plan.ngroups + sms - 1) / sms), ring = tile_by_rows<BS, TS>() ? 8 : 4;
   int c = want, nslot = tile_slots<BS, TS>(gmax, nlev_max, c, optin);

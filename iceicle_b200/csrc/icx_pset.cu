@@ -258,7 +258,8 @@ icx_status ensure_buffers(icx_pset* S, int m) {
 cudaError_t seg_dots(icx_pset* S, const double* V, long long ld, int nvec, const double* x, double* out, int ldo,
                      cudaStream_t s) {
   const int ldp = S->m + 2;
-  seg_dot_partial_kernel<<<dim3(S->n_chunks, std::min(nvec, kSplit)), kThreads, 0, s>>>(S->d_cbeg, S->d_cend, V, ld, nvec, x, S->partial, ldp);
+  seg_dot_partial_kernel<<<dim3(S->n_chunks, std::min(nvec, kSplit)), kThreads, 0, s>>>(S->d_cbeg, S->d_cend, V, ld,
+                                                                                        nvec, x, S->partial, ldp);
   seg_dot_final_kernel<<<(S->n_parts + 7) / 8, 256, 0, s>>>(S->n_parts, S->d_pck, S->partial, ldp, nvec, out, ldo);
   return cudaGetLastError();
 }
@@ -487,8 +488,8 @@ icx_status pset_gmres(icx_pset* S, int pc, bool mixed, int m, int maxit, double 
     PCK(cudaMemcpyAsync(S->coef, S->h_small, sizeof(double) * P * ld, cudaMemcpyHostToDevice, s));
     PCK(cudaMemsetAsync(S->w, 0, sizeof(double) * N, s));
     if (jmax > 0) {
-      seg_maxpy_kernel<<<dim3(S->n_chunks, kSplit), kThreads, 0, s>>>(S->d_cbeg, S->d_cend, S->d_cpart, S->V, N, jmax, S->coef, ld,
-                                                       1.0, S->w);
+      seg_maxpy_kernel<<<dim3(S->n_chunks, kSplit), kThreads, 0, s>>>(S->d_cbeg, S->d_cend, S->d_cpart, S->V, N, jmax,
+                                                                      S->coef, ld, 1.0, S->w);
       PCK(cudaGetLastError());
     }
     if (pc) {

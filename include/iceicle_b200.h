@@ -311,9 +311,8 @@ typedef struct icx_newton_options {
    * linearisations: its residual, norm, line search and update stay FP64.
    * 3: as 1, with the block-ILU(0) factors of a tiled or grouped
    * preconditioner (ilu_tile, icx_set_ilu_groups) stored in BF16 and widened
-   * to FP32 in the apply (the one-lane-per-row form, ilu_sched 5; where its
-   * shared memory does not fit, and on whole-grid factors, the FP32 copies
-   * of 1). The preconditioner only changes GMRES iterations: the converged
+   * to FP32 in the apply (ilu_sched 5; where its shared memory does not fit,
+   * and on whole-grid factors, the FP32 copies of 1). The preconditioner only changes GMRES iterations: the converged
    * state is judged in FP64 as in 1. */
   int precision;
   /* preconditioner 4 (block-ILU(0) factors applied by Jacobi sweeps): the
@@ -621,14 +620,18 @@ icx_status icx_basis_node_coords(const icx_ctx* ctx, double* xy);
  *               SM of the persistent grid (1 to 4; capped by occupancy) and the
  *               schedule: 1 completion counters per element, 2 outputs
  *               pre-filled with a sentinel and polled directly (the default
- *               on whole-grid factors), 3 on tiled or grouped factors one CTA
+ *               on whole-grid factors; at the default rows and CTAs a whole
+ *               structured grid runs by strips of its rows, same results), 3 on tiled or grouped factors one CTA
  *               per tile running the tile's levels between CTA barriers, 4 the
  *               same with each warp's next task rows copied ahead into shared
  *               memory, 5 one lane per matrix row with the tile's vectors in
  *               shared memory (the defaults there: 5 for FP32 factors, 4 for
- *               FP64 ones; each falls back to the one
- *               below where its shared memory does not fit; 3 to 5 are 2 on
- *               whole-grid factors; 5 sums each row's columns in order, so
+ *               FP64 ones; at the default shape of 4 in FP64, and at every
+ *               shape of 5 in FP32 and BF16, the factors are streamed through
+ *               shared memory where the block size and the tile allow; each
+ *               falls back to the one below where its shared memory does not
+ *               fit; 3 to 5 are 2 on whole-grid factors; 5 sums a row's
+ *               columns in another order where it does not stream, so
  *               its results differ from the others' in rounding); for 3 to 5
  *               ilu_ctas picks the threads per CTA instead: 0 the default
  *               (256 FP64, 512 FP32 factors), 1 / 2 / 3 512 / 256 / 128 */

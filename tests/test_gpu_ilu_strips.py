@@ -1,7 +1,7 @@
 """The block-ILU(0) apply by strips of grid rows (the default on whole grids for
 blocks up to 36 x 36) against the data-flow apply on completion counters: the
 same sums in the same order, so the results are equal bit for bit. Sizes: one
-row, one column, fewer rows than a strip, ragged last strips, more strips than
+row, one column, fewer rows than a strip, ragged last strips, wide rows, more strips than
 a cluster and more than are resident at once; batches of grids; both
 precisions; repeated applies (the exchange rows are left ready for the next)."""
 import numpy as np
@@ -17,7 +17,8 @@ pytestmark = pytest.mark.gpu
 CASES = [dict(pde=BURGERS, p=p, g=1, nx=nx, ny=ny) for p in (1, 2, 3, 4)
          for nx, ny in ((1, 1), (1, 19), (23, 1), (7, 5), (12, 33), (3, 90))]
 CASES += [dict(pde=NS, p=1, g=1, nx=9, ny=14), dict(pde=NS, p=2, g=1, nx=5, ny=20),
-          dict(pde=NS, p=2, g=1, nx=2, ny=300)]
+          dict(pde=NS, p=2, g=1, nx=2, ny=300),
+          dict(pde=NS, p=2, g=1, nx=400, ny=3)]  # rows too wide for an inbox
 
 
 def check(ctx, n, precision):
