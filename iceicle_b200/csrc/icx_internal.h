@@ -243,6 +243,8 @@ const float* solver_vals32(icx_ctx* c);
 // solver_prepare_pc with kind 2), and the apply's error flag (read, then
 // cleared with the completion counters when set)
 cudaError_t solver_apply_ilu_flow(icx_ctx* c, bool mixed, const double* x, double* z, cudaStream_t s);
+// the whole-grid apply's packed factors of one precision, from the factors in place, at the context's tile choice
+cudaError_t solver_pack_strips(icx_ctx* c, bool mixed, cudaStream_t s);
 icx_status solver_take_pc_err(icx_ctx* c, int* err);
 // the per-group pieces of a batch of independent solves (icx_pset.cu):
 // buffers and options, the FP64 residual with the Jacobian (precision 2: FP32

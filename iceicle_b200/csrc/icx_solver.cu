@@ -482,6 +482,24 @@ bool strip_shape(const icx_ctx* c, bool mixed) {
          (t.flow_ctas[pi] == 0 || t.flow_ctas[pi] == 2);
 }
 
+// packs the current factors for the strip apply of one precision, where it runs; without the memory for them the
+// data-flow apply stays
+cudaError_t pack_strips(icx_ctx* c, bool mixed, cudaStream_t s) {
+  icx_solver_work* w = c->sw;
+  const int pi = mixed ? 1 : 0;
+  w->sp_ok[pi] = false;
+  if (!strip_shape(c, mixed)) return cudaSuccess;
+  if (!w->spk[pi] && cudaMalloc(&w->spk[pi], (size_t)w->sp[pi].bytes) != cudaSuccess) {
+    (void)cudaGetLastError();
+    w->spk[pi] = nullptr;
+    return cudaSuccess;
+  }
+  const cudaError_t e = mixed ? icx::la_ilu_strip_pack_f32(w->bs, w->sp[1], w->pc, w->uinv, (float*)w->spk[1], s)
+                              : icx::la_ilu_strip_pack(w->bs, w->sp[0], w->pc, w->uinv, (double*)w->spk[0], s);
+  w->sp_ok[pi] = e == cudaSuccess;
+  return e;
+}
+
 // the data-flow block-ILU(0) apply with the context's launch shape. Each
 // apply adds an element's task count to its counters and waits for
 // epoch x task count, so a change of rows per task (FP64 and FP32 applies may
@@ -637,14 +655,7 @@ cudaError_t build_pc_impl(icx_ctx* c, int kind, bool mixed, cudaStream_t s) {
   }
   // the strips' packed factors (kind 4 applies its factors by other kernels)
   w->sp_ok[0] = w->sp_ok[1] = false;
-  const int pi = mixed ? 1 : 0;
-  if (e == cudaSuccess && ilu && kind != 4 && strip_shape(c, mixed)) {
-    if (!w->spk[pi]) e = cudaMalloc(&w->spk[pi], (size_t)w->sp[pi].bytes);
-    if (e == cudaSuccess)
-      e = mixed ? icx::la_ilu_strip_pack_f32(w->bs, w->sp[1], w->pc, w->uinv, (float*)w->spk[1], s)
-                : icx::la_ilu_strip_pack(w->bs, w->sp[0], w->pc, w->uinv, (double*)w->spk[0], s);
-    w->sp_ok[pi] = e == cudaSuccess;
-  }
+  if (e == cudaSuccess && ilu && kind != 4) e = pack_strips(c, mixed, s);
   if (e != cudaSuccess || !mixed) return e;
   e = icx::la_d2f(nv, w->vals, w->vals32, s);
   if (e == cudaSuccess && jac) e = icx::la_d2f(nd, w->pc, w->pc32, s);
@@ -1312,6 +1323,8 @@ icx_status solver_prepare_pc(icx_ctx* c, const double* vals, int kind, int sweep
 cudaError_t solver_apply_pc(icx_ctx* c, int kind, bool mixed, const double* x, double* z, cudaStream_t s) {
   return apply_pc(c, kind, mixed, x, z, s);
 }
+
+cudaError_t solver_pack_strips(icx_ctx* c, bool mixed, cudaStream_t s) { return pack_strips(c, mixed, s); }
 
 const float* solver_vals32(icx_ctx* c) { return c->sw ? c->sw->vals32 : nullptr; }
 

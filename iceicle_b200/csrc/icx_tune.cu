@@ -215,6 +215,7 @@ struct Tuner {
         return ICX_OK;
       };
       dm.tile.flow_rows[pi] = dm.tile.flow_ctas[pi] = dm.tile.flow_sched[pi] = 0;
+      TCK(icx::solver_pack_strips(c, mixed, s));  // the default is timed as the solves run it
       TCK(apply(z0));
       TCK(cudaStreamSynchronize(s));
       if ((st = check_err()) != ICX_OK) { dm.tile = keep; return st; }
