@@ -101,6 +101,16 @@ __device__ inline double ld_cluster_f64(unsigned addr) {
 constexpr int kStripCheck = 16;
 __device__ inline bool strip_check(int t, int nsteps) { return t % kStripCheck == kStripCheck - 1 || t == nsteps - 1; }
 
+// all bits set: a NaN in FP64, and two of them in FP32
+__device__ inline double strip_nan() { return __longlong_as_double(-1ll); }
+
+// y of a strip whose sweeps were given up: NaN, never what y held before or values of an unfinished sweep
+template <int BS>
+__device__ inline void strip_give_up(const IluStrip& st, double* y) {
+  double* const ys = y + ((size_t)st.e0 + (size_t)st.j0 * st.nx) * BS;
+  for (int i = threadIdx.x; i < st.nr * st.nx * BS; i += blockDim.x) ys[i] = strip_nan();
+}
+
 template <int BS, class TA>
 struct StripShared {
   double vec[2][StripCfg<BS, TA>::S + 1][BS];  // by step parity: the neighbour strip's element, then each row's
@@ -141,6 +151,12 @@ __device__ inline bool strip_sweep(const StripArgs<TA>& a, int s, StripShared<BS
       for (int p = 0; p < NP; ++p)
         if (has_prev && !near && c < nx && lane + 32 * p < BS) o[p] = ld_relaxed_f64(ein + (size_t)c * BS + lane + 32 * p);
     };
+    // given up: a NaN in the neighbour's row from here on, so that what is still computed and handed on cannot pass
+    // for a result (an element's rows all read all of its neighbours; the step that is running may or may not see it)
+    auto poison = [&]() {
+      if (lane < 2) *reinterpret_cast<volatile double*>(sh.vec[lane][0]) = strip_nan();
+      return false;
+    };
     // element c's vector (slot u0 of the window c .. c + Q - 1) into shared memory; false when the wait was
     // given up. A wait asks again for the whole window: a poll's trip covers several of the producer's steps,
     // and a window asked for element by element would cost a trip for each
@@ -167,7 +183,7 @@ __device__ inline bool strip_sweep(const StripArgs<TA>& a, int s, StripShared<BS
               quit = 1;
             }
           }
-          if (__shfl_sync(0xffffffffu, quit, 0)) return false;
+          if (__shfl_sync(0xffffffffu, quit, 0)) return poison();
         }
 #pragma unroll
         for (int p = 0; p < NP; ++p)
@@ -191,7 +207,7 @@ __device__ inline bool strip_sweep(const StripArgs<TA>& a, int s, StripShared<BS
             quit = 1;
           }
         }
-        if (__shfl_sync(0xffffffffu, quit, 0)) return false;
+        if (__shfl_sync(0xffffffffu, quit, 0)) return poison();
 #pragma unroll
         for (int d = 0; d < Q; ++d) ask(c + d, v[(u0 + d) % Q]);
       }
@@ -206,7 +222,7 @@ __device__ inline bool strip_sweep(const StripArgs<TA>& a, int s, StripShared<BS
 #pragma unroll
     for (int u = 0; u < Q; ++u) ask(u, v[u]);
     // an apply that was given up leaves *err set: later ones end at once
-    bool ok = *reinterpret_cast<volatile int*>(a.err) == 0;
+    bool ok = __all_sync(0xffffffffu, *reinterpret_cast<volatile int*>(a.err) == 0) || poison();
     ok = ok && take(0, 0, sh.vec[1][0]);
     ask(Q, v[0]);
     __syncthreads();
@@ -245,7 +261,11 @@ __device__ inline bool strip_sweep(const StripArgs<TA>& a, int s, StripShared<BS
       islot = islot + 1 == D ? 0 : islot + 1;
     };
     auto wait = [&]() {
-      if (waited < nch && !mbar_wait(bar0 + 8 * wslot, phase)) ok = false;
+      if (!__all_sync(0xffffffffu, waited >= nch || mbar_wait(bar0 + 8 * wslot, phase))) {
+        // not landed: NaN in its place (a copy that lands after all brings the right entries)
+        ok = false;
+        for (int i = lane; i < K::CHUNK / 8; i += 32) reinterpret_cast<double*>(ring + wslot * K::CHUNK)[i] = strip_nan();
+      }
       ++waited;
       if (++wslot == D) {
         wslot = 0;
@@ -454,10 +474,15 @@ __global__ void __launch_bounds__((StripCfg<BS, TA>::NT)) ilu_apply_strip_kernel
   bool ok = true;
   if (a.sweep == 0) {
     for (; ok && s < a.nstrips; s += gridDim.x) ok = strip_sweep<BS, TA, true>(a, s, sh, ring, inbox, gch);
-    for (s -= gridDim.x; ok && s >= 0; s -= gridDim.x) ok = strip_sweep<BS, TA, false>(a, s, sh, ring, inbox, gch);
+    while (s < a.nstrips) s += gridDim.x;  // given up forwards: none of this CTA's strips is finished
+    for (s -= gridDim.x; s >= 0; s -= gridDim.x) {
+      ok = ok && strip_sweep<BS, TA, false>(a, s, sh, ring, inbox, gch);
+      if (!ok) strip_give_up<BS>(a.strips[s], a.y);
+    }
   } else if (s < a.nstrips) {
+    // the backward launch after a forward one that was given up ends at once (*err)
     if (a.sweep == 1) strip_sweep<BS, TA, true>(a, s, sh, ring, inbox, gch);
-    else strip_sweep<BS, TA, false>(a, s, sh, ring, inbox, gch);
+    else if (!strip_sweep<BS, TA, false>(a, s, sh, ring, inbox, gch)) strip_give_up<BS>(a.strips[s], a.y);
   }
   // no CTA of a cluster ends while another may still store into its inbox
   if (a.cluster > 1) cluster_sync();
