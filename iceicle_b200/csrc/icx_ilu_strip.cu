@@ -49,6 +49,9 @@ struct StripCfg {
   static constexpr int NL = S * EL;                  // lanes with work
   static constexpr int NW = (NL + 31) / 32;          // worker warps
   static constexpr int NT = NW * 32 + 96;            // and the fetcher, the loader and the vector warp
+  // CTAs per SM to compile for: what sets of problems side by side share an SM with (16 x 16 blocks compiled for one:
+  // a set of 16 problems, orders 1 to 4, 314 ms instead of 301; left to the compiler 304)
+  static constexpr int MINB = BS == 4 ? 4 : BS == 9 || BS == 16 ? 2 : 1;
   static constexpr int NF = 2 * NCOL, NB = 3 * NCOL; // entries per lane and step, forward and backward
   static constexpr int BF = (NF * NL * (int)sizeof(TA) + 15) / 16 * 16;  // bytes of a packed step
   static constexpr int BB = (NB * NL * (int)sizeof(TA) + 15) / 16 * 16;
@@ -69,11 +72,13 @@ struct StripArgs {
   int* err;
   int depth;   // chunks in the ring
   int cluster; // CTAs per cluster (1: every hand-over through the exchange rows)
+  int inbox;   // values of an inbox: a row of the widest grid (the same in all CTAs of a cluster)
   int sweep;   // 0 both sweeps in one launch (all CTAs resident), 1 the forward one, 2 the backward one
   unsigned long long* ticket;  // sweep 1 and 2: tickets drawn by the clusters so far
 };
 
-// a row handed over inside a cluster goes straight into the consumer's shared memory
+// a row handed over inside a cluster goes straight into the consumer's shared memory, into an inbox per sweep of the
+// launch: a slot is written once, so no store of the backward sweep has to be ordered against the forward one's
 __device__ inline unsigned cluster_rank() {
   unsigned r;
   asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
@@ -187,10 +192,7 @@ __device__ inline bool strip_sweep(const StripArgs<TA>& a, int s, StripShared<BS
         }
 #pragma unroll
         for (int p = 0; p < NP; ++p)
-          if (lane + 32 * p < BS) {
-            dst[lane + 32 * p] = o[p];
-            inbox[c * BS + lane + 32 * p] = __longlong_as_double((long long)FLOW_SENTINEL);
-          }
+          if (lane + 32 * p < BS) dst[lane + 32 * p] = o[p];
         return true;
       }
       while (true) {
@@ -444,7 +446,7 @@ __device__ inline bool strip_sweep(const StripArgs<TA>& a, int s, StripShared<BS
 // than the GPU, and for several applies side by side (cooperative launches run
 // one after the other).
 template <int BS, class TA>
-__global__ void __launch_bounds__((StripCfg<BS, TA>::NT)) ilu_apply_strip_kernel(StripArgs<TA> a) {
+__global__ void __launch_bounds__((StripCfg<BS, TA>::NT), (StripCfg<BS, TA>::MINB)) ilu_apply_strip_kernel(StripArgs<TA> a) {
   using K = StripCfg<BS, TA>;
   extern __shared__ __align__(128) unsigned char ring[];
   __shared__ StripShared<BS, TA> sh;
@@ -464,7 +466,7 @@ __global__ void __launch_bounds__((StripCfg<BS, TA>::NT)) ilu_apply_strip_kernel
     s = (int)(a.sweep == 1 ? t : ncl - 1 - t) * a.cluster + (int)cluster_rank();
   }
   if (a.cluster > 1) {
-    const int n = s < a.nstrips ? a.strips[s].nx * BS : 0;
+    const int n = a.sweep == 0 ? 2 * a.inbox : a.inbox;
     for (int i = threadIdx.x; i < n; i += K::NT) inbox[i] = __longlong_as_double((long long)FLOW_SENTINEL);
     cluster_sync();
   } else {
@@ -476,7 +478,7 @@ __global__ void __launch_bounds__((StripCfg<BS, TA>::NT)) ilu_apply_strip_kernel
     for (; ok && s < a.nstrips; s += gridDim.x) ok = strip_sweep<BS, TA, true>(a, s, sh, ring, inbox, gch);
     while (s < a.nstrips) s += gridDim.x;  // given up forwards: none of this CTA's strips is finished
     for (s -= gridDim.x; s >= 0; s -= gridDim.x) {
-      ok = ok && strip_sweep<BS, TA, false>(a, s, sh, ring, inbox, gch);
+      ok = ok && strip_sweep<BS, TA, false>(a, s, sh, ring, inbox + a.inbox, gch);
       if (!ok) strip_give_up<BS>(a.strips[s], a.y);
     }
   } else if (s < a.nstrips) {
@@ -534,7 +536,7 @@ template <int BS, class TA>
 cudaError_t launch_strips(const IluStripPlan& p, const StripArgs<TA>& args, bool side_by_side, cudaStream_t s) {
   using K = StripCfg<BS, TA>;
   constexpr auto kern = ilu_apply_strip_kernel<BS, TA>;
-  constexpr int kSmem = 224 * 1024, kCluster = 8;
+  constexpr int kSmem = 225 * 1024, kCluster = 8;
   int dev = 0, nsm = 0;
   cudaError_t e = cudaGetDevice(&dev);
   if (e == cudaSuccess) e = cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
@@ -542,13 +544,12 @@ cudaError_t launch_strips(const IluStripPlan& p, const StripArgs<TA>& args, bool
   StripArgs<TA> a = args;
   // clusters of strips that hand their rows over in shared memory, where the inbox (a row of the widest grid)
   // leaves room for two chunks; side by side with other applies no more than two, so that several CTAs share an SM
-  const long long inbox = (long long)p.max_nx * BS * 8;
-  const long long fit = (kSmem - K::VD * K::VB - inbox) / K::CHUNK;
-  if (fit >= 2) {
-    a.depth = (int)std::min<long long>(side_by_side ? 2 : 4, fit);
+  a.inbox = p.max_nx * BS;
+  const long long inbox = (long long)a.inbox * 8;
+  const auto fit = [&](int inboxes) { return (kSmem - K::VD * K::VB - inboxes * inbox) / K::CHUNK; };
+  if (fit(1) >= 2) {
     cudaLaunchConfig_t cfg = {};
     cfg.blockDim = dim3(K::NT);
-    cfg.dynamicSmemBytes = (size_t)a.depth * K::CHUNK + K::VD * K::VB + inbox;
     cfg.stream = s;
     cudaLaunchAttribute attr[2];
     attr[0].id = cudaLaunchAttributeClusterDimension;
@@ -556,22 +557,32 @@ cudaError_t launch_strips(const IluStripPlan& p, const StripArgs<TA>& args, bool
     attr[1].id = cudaLaunchAttributeCooperative;
     attr[1].val.cooperative = 1;
     cfg.attrs = attr;
-    e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)cfg.dynamicSmemBytes);
-    if (e != cudaSuccess) return e;
     cfg.gridDim = dim3((p.nstrips + kCluster - 1) / kCluster * kCluster);
     attr[0].val.clusterDim.x = a.cluster = kCluster;
-    cfg.numAttrs = 1;
     int clusters = 0;
-    if (cudaOccupancyMaxActiveClusters(&clusters, kern, &cfg) != cudaSuccess) {
-      (void)cudaGetLastError();
-      clusters = 0;
+    const auto size = [&](int inboxes) {
+      a.depth = (int)std::min<long long>(side_by_side ? 2 : 4, fit(inboxes));
+      cfg.dynamicSmemBytes = (size_t)a.depth * K::CHUNK + K::VD * K::VB + inboxes * inbox;
+      cfg.numAttrs = 1;
+      const cudaError_t er = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                                  (int)cfg.dynamicSmemBytes);
+      if (er == cudaSuccess && cudaOccupancyMaxActiveClusters(&clusters, kern, &cfg) != cudaSuccess) {
+        (void)cudaGetLastError();
+        clusters = 0;
+      }
+      return er;
+    };
+    // one cooperative launch for both sweeps (saves a launch and the tickets) where their inboxes leave the ring three
+    // chunks, or as many as one inbox does, and the whole grid is resident
+    if (!side_by_side && fit(2) >= std::min<long long>(3, fit(1))) {
+      if ((e = size(2)) != cudaSuccess) return e;
+      if ((long long)clusters * kCluster >= cfg.gridDim.x) {
+        cfg.numAttrs = 2;
+        a.sweep = 0;
+        return cudaLaunchKernelEx(&cfg, kern, a);
+      }
     }
-    // one cooperative launch for both sweeps where the whole grid is resident (saves a launch and the tickets)
-    if (!side_by_side && (long long)clusters * kCluster >= cfg.gridDim.x) {
-      cfg.numAttrs = 2;
-      a.sweep = 0;
-      return cudaLaunchKernelEx(&cfg, kern, a);
-    }
+    if ((e = size(1)) != cudaSuccess) return e;
     if (clusters > 0) {
       for (a.sweep = 1; a.sweep <= 2; ++a.sweep)
         if ((e = cudaLaunchKernelEx(&cfg, kern, a)) != cudaSuccess) return e;
@@ -606,7 +617,7 @@ template <class TA>
 cudaError_t apply_strips(int bs, const IluStripPlan& p, const TA* pk, const double* x, double* y, double* f, int* err,
                          bool side_by_side, cudaStream_t s) {
   if (p.nstrips < 1 || !pk) return cudaErrorInvalidValue;
-  StripArgs<TA> a{p.nstrips, p.strips, reinterpret_cast<const unsigned char*>(pk), x, f, y, p.ex, err, 0, 1, 0, p.ticket};
+  StripArgs<TA> a{p.nstrips, p.strips, reinterpret_cast<const unsigned char*>(pk), x, f, y, p.ex, err, 0, 1, 0, 0, p.ticket};
 #define ICX_STRIP_CASE(B) \
   if (bs == B) return launch_strips<B, TA>(p, a, side_by_side, s);
   ICX_STRIP_SIZES(ICX_STRIP_CASE)
