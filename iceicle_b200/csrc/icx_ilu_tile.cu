@@ -34,8 +34,9 @@
 // for a slot's previous element, whose warp waits for no later element. The
 // waits are bounded all the same (ICX_FLOW_SPINS): *err = 1, and a warp that
 // gave up goes on through the same barriers without computing and gives no
-// slot back, so nothing is filled under another's feet. The producer leaves
-// only after its last copies have landed.
+// slot back, so nothing is filled under another's feet; y of its group is NaN
+// then, never what it held before. The producer leaves only after its last
+// copies have landed.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -189,6 +190,7 @@ struct TileCta {
 struct TileShared {
   int slev[kGroupLevelsSmem + 1];
   int held[kTileSlotsMax];  // the element of the order of use that a slot is being filled with
+  int gave_up;              // a wait ran out
   unsigned long long bars[2 * kTileSlotsMax];
 };
 
@@ -235,6 +237,7 @@ __device__ inline bool tile_setup(const IluGroupArgs<TS>& a, int nslot, TileShar
       for (int k = lane * 16; k < BS; k += 512)
         asm volatile("prefetch.global.L2 [%0];" ::"l"(a.x + (size_t)e * BS + k));
   }
+  if (threadIdx.x == 0) sh.gave_up = 0;
   if (threadIdx.x < nslot) {
     sh.held[threadIdx.x] = -1;
     mbar_init(c.full + 8 * threadIdx.x, 1);
@@ -287,6 +290,15 @@ __device__ inline bool tile_wait(const TileShared& sh, unsigned full, int slot, 
   unsigned spins = 0;
   while (*(const volatile int*)(sh.held + slot) != n && ++spins < ICX_FLOW_SPINS) {}
   return spins < ICX_FLOW_SPINS && mbar_wait(full + 8 * slot, parity);
+}
+
+// y of a group that was given up, by NT threads after their last barrier
+template <int BS, class TS>
+__device__ inline void tile_give_up(const IluGroupArgs<TS>& a, const TileCta<TS>& c, int nt) {
+  for (int i = threadIdx.x; i < c.G * BS; i += nt) {
+    const int e = c.tab[i / BS].x;
+    if (e >= 0) a.y[(size_t)e * BS + i % BS] = __longlong_as_double(-1ll);
+  }
 }
 
 // a warp per element, eight rows at a time
@@ -347,7 +359,10 @@ __global__ void __launch_bounds__(NW * 32 + 32, MINB) ilu_apply_tile_kernel(IluG
       if (!__all_sync(0xffffffffu, ready) && ok) {
         ok = tile_wait(sh, full, slot, m, (unsigned)t.z >> 24);
         ok = __all_sync(0xffffffffu, ok);
-        if (!ok && lane == 0) atomicExch(a.err, 1);
+        if (!ok && lane == 0) {
+          atomicExch(a.err, 1);
+          sh.gave_up = 1;
+        }
       }
       if (ok && t.x >= 0) {
         const TS* A = reinterpret_cast<const TS*>(cta.ring + (size_t)slot * K::SLOT);
@@ -382,6 +397,7 @@ __global__ void __launch_bounds__(NW * 32 + 32, MINB) ilu_apply_tile_kernel(IluG
     }
     asm volatile("bar.sync 1, %0;" ::"n"(NW * 32) : "memory");
   }
+  if (sh.gave_up) tile_give_up<BS, TS>(a, cta, NW * 32);
 }
 
 // BF16 factors, rows of half-bank stride (BS = 36): a thread per matrix row,
@@ -516,6 +532,7 @@ __global__ void __launch_bounds__(TileRowCfg<BS>::NT + 32, 2)
     }
     if (ok && m >= 0 && r == 0) mbar_arrive(cta.empty + 8 * slot);
   }
+  if (!ok) tile_give_up<BS, TS>(a, cta, R::NT);
 }
 
 // slots of the ring with `ctas` CTAs on an SM; fewer than three: not by this kernel
