@@ -115,7 +115,8 @@ cudaError_t ilu_apply_groups_t(const DeviceMesh& dm, const IluGroupShape& gs, co
 #undef ICX_ILUG_CASE
   if (!k.kern) return cudaErrorInvalidValue;
   if (k.smem > 48 * 1024) {
-    cudaError_t e = cudaFuncSetAttribute(k.kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)k.smem);
+    // the limit is a property of the kernel, shared by all threads: always the same value
+    cudaError_t e = cudaFuncSetAttribute(k.kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_avail());
     if (e != cudaSuccess) return e;
   }
   IluGroupArgs<TA> args{dm.E, dm.nnzb, LU, Uinv, x, f, y, err,
@@ -141,7 +142,8 @@ cudaError_t la_ilu_apply_groups_bf16(const DeviceMesh& dm, const IluGroupShape& 
 #undef ICX_ILUG16_CASE
   if (!k.kern) return cudaErrorNotSupported;  // the one-lane-per-row form does not fit
   if (k.smem > 48 * 1024) {
-    cudaError_t e = cudaFuncSetAttribute(k.kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)k.smem);
+    // the limit is a property of the kernel, shared by all threads: always the same value
+    cudaError_t e = cudaFuncSetAttribute(k.kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_avail());
     if (e != cudaSuccess) return e;
   }
   IluGroupArgs<__nv_bfloat16> args{dm.E, dm.nnzb, LU, Uinv, x, f, y, err,

@@ -540,6 +540,8 @@ cudaError_t launch_strips(const IluStripPlan& p, const StripArgs<TA>& args, bool
   int dev = 0, nsm = 0;
   cudaError_t e = cudaGetDevice(&dev);
   if (e == cudaSuccess) e = cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
+  // the limit is a property of the kernel, shared by all threads: always the same value
+  if (e == cudaSuccess) e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmem);
   if (e != cudaSuccess) return e;
   StripArgs<TA> a = args;
   // clusters of strips that hand their rows over in shared memory, where the inbox (a row of the widest grid)
@@ -564,25 +566,22 @@ cudaError_t launch_strips(const IluStripPlan& p, const StripArgs<TA>& args, bool
       a.depth = (int)std::min<long long>(side_by_side ? 2 : 4, fit(inboxes));
       cfg.dynamicSmemBytes = (size_t)a.depth * K::CHUNK + K::VD * K::VB + inboxes * inbox;
       cfg.numAttrs = 1;
-      const cudaError_t er = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                                  (int)cfg.dynamicSmemBytes);
-      if (er == cudaSuccess && cudaOccupancyMaxActiveClusters(&clusters, kern, &cfg) != cudaSuccess) {
+      if (cudaOccupancyMaxActiveClusters(&clusters, kern, &cfg) != cudaSuccess) {
         (void)cudaGetLastError();
         clusters = 0;
       }
-      return er;
     };
     // one cooperative launch for both sweeps (saves a launch and the tickets) where their inboxes leave the ring three
     // chunks, or as many as one inbox does, and the whole grid is resident
     if (!side_by_side && fit(2) >= std::min<long long>(3, fit(1))) {
-      if ((e = size(2)) != cudaSuccess) return e;
+      size(2);
       if ((long long)clusters * kCluster >= cfg.gridDim.x) {
         cfg.numAttrs = 2;
         a.sweep = 0;
         return cudaLaunchKernelEx(&cfg, kern, a);
       }
     }
-    if ((e = size(1)) != cudaSuccess) return e;
+    size(1);
     if (clusters > 0) {
       for (a.sweep = 1; a.sweep <= 2; ++a.sweep)
         if ((e = cudaLaunchKernelEx(&cfg, kern, a)) != cudaSuccess) return e;
@@ -595,9 +594,7 @@ cudaError_t launch_strips(const IluStripPlan& p, const StripArgs<TA>& args, bool
   a.sweep = 0;
   const size_t smem = (size_t)a.depth * K::CHUNK + K::VD * K::VB;
   int per_sm = 0;
-  e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-  if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, K::NT, smem);
-  if (e != cudaSuccess) return e;
+  if ((e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, K::NT, smem)) != cudaSuccess) return e;
   if (per_sm < 1 || a.depth < 2) return cudaErrorNotSupported;
   const int grid = std::min(p.nstrips, nsm * per_sm);
   void* params[] = {&a};

@@ -582,7 +582,9 @@ cudaError_t tile_launch(const IluGroupArgs<TS>& args, int nlev_max, cudaStream_t
     nt = 4 * 32 + 32;
   }
   const size_t smem = (size_t)nslot * K::SLOT + tile_fixed_smem<BS, TS>(gmax);
-  const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  // the limit is a property of the kernel, shared by all threads: always the same value (tile_slots leaves 2048 bytes
+  // to the static shared memory)
+  const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, optin - 2048);
   if (e != cudaSuccess) return e;
   IluGroupArgs<TS> ka = args;
   void* params[] = {&ka, &nslot};
