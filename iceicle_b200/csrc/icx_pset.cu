@@ -33,6 +33,7 @@
 #include <string>
 #include <vector>
 
+#include "icx_forks.h"
 #include "icx_internal.h"
 #include "icx_linalg.h"
 
@@ -191,9 +192,7 @@ struct icx_pset {
   double* h_hcol = nullptr;           // pinned copy of hcol
   double* h_small = nullptr;          // pinned [n_parts][m + 2] staging
   cudaStream_t cap = nullptr;         // graph capture stream
-  std::vector<cudaStream_t> side;     // all_groups: a stream per group but the last, its completion, the fork
-  std::vector<cudaEvent_t> joined;
-  cudaEvent_t forked = nullptr;
+  icx::Forks<icx::CudaForks> forks;   // all_groups: streams for the groups side by side
   std::vector<cudaGraphExec_t> exec;  // Arnoldi step graphs (step j)
   std::vector<int> seen;
   unsigned long long key = 0;
@@ -282,39 +281,15 @@ cudaError_t put_per_part(icx_pset* S, const std::vector<double>& v, double* dst,
 }
 
 // f for every group, the groups side by side: the last (the highest order, the
-// longest) on stream q, the others on side streams that start after q's work so
-// far and that q then waits for. The groups' buffers are their own and their
-// parts of the set's vectors do not overlap; their launches are bound by latency
-// (the block-ILU(0) apply above all) and leave most of the GPU to one another:
-// set of 16 problems, orders 1 to 4, 603 ms in turn, 351 ms side by side. Works the same
-// under stream capture (the fork and the join become edges of the graph).
+// longest) on stream q, the others on side streams. The groups' buffers are
+// their own and their parts of the set's vectors do not overlap; their launches
+// are bound by latency (the block-ILU(0) apply above all) and leave most of the
+// GPU to one another: set of 16 problems, orders 1 to 4, 603 ms in turn, 351 ms
+// side by side
 cudaError_t all_groups(icx_pset* S, cudaStream_t q,
                        const std::function<cudaError_t(icx_ctx*, long long, cudaStream_t)>& f) {
-  const size_t n = S->groups.size();
-  cudaError_t e = cudaSuccess;
-  while (e == cudaSuccess && S->side.size() + 1 < n) {
-    cudaStream_t t = nullptr;
-    cudaEvent_t ev = nullptr;
-    if ((e = cudaStreamCreateWithFlags(&t, cudaStreamNonBlocking)) != cudaSuccess) break;
-    S->side.push_back(t);
-    if ((e = cudaEventCreateWithFlags(&ev, cudaEventDisableTiming)) == cudaSuccess) S->joined.push_back(ev);
-  }
-  if (e == cudaSuccess && n > 1 && !S->forked) e = cudaEventCreateWithFlags(&S->forked, cudaEventDisableTiming);
-  if (e == cudaSuccess && n > 1) e = cudaEventRecord(S->forked, q);
-  size_t begun = 0;
-  for (size_t g = 0; g + 1 < n && e == cudaSuccess; ++g) {
-    if ((e = cudaStreamWaitEvent(S->side[g], S->forked, 0)) != cudaSuccess) break;
-    ++begun;
-    e = f(S->groups[g], S->group_off[g], S->side[g]);
-  }
-  if (e == cudaSuccess && n > 0) e = f(S->groups[n - 1], S->group_off[n - 1], q);
-  // every stream begun is joined, also after an error
-  for (size_t g = 0; g < begun; ++g) {
-    cudaError_t j = cudaEventRecord(S->joined[g], S->side[g]);
-    if (j == cudaSuccess) j = cudaStreamWaitEvent(q, S->joined[g], 0);
-    if (e == cudaSuccess) e = j;
-  }
-  return e;
+  return S->forks.run(S->groups.size(), q,
+                      [&](size_t g, cudaStream_t t) { return f(S->groups[g], S->group_off[g], t); });
 }
 
 struct Kry {
@@ -613,9 +588,7 @@ void icx_pset_destroy(icx_pset* S) {
   cudaSetDevice(S->device);
   free_buffers(S);
   if (S->cap) cudaStreamDestroy(S->cap);
-  for (cudaStream_t t : S->side) cudaStreamDestroy(t);
-  for (cudaEvent_t ev : S->joined) cudaEventDestroy(ev);
-  if (S->forked) cudaEventDestroy(S->forked);
+  S->forks.release();
   void* dev[] = {S->d_cbeg, S->d_cend, S->d_cpart, S->d_pck};
   for (void* p : dev)
     if (p) cudaFree(p);
