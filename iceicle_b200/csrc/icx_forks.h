@@ -60,21 +60,28 @@ class Forks {
     forked = nullptr;
   }
 
-  // f(k, stream) for k < n: the last on q, the others on side streams that q
-  // then waits for. Works the same under stream capture (fork and join become
-  // edges of the graph).
-  template <class F>
-  cudaError_t run(size_t n, cudaStream_t q, const F& f) {
+  // f(k, stream) for k < n: the pieces for which alone(k) holds on q, one after
+  // the other (the last piece where it holds for none), the others on side
+  // streams that q then waits for. Works the same under stream capture (fork
+  // and join become edges of the graph).
+  template <class A, class F>
+  cudaError_t run(size_t n, cudaStream_t q, const A& alone, const F& f) {
     if (n == 0) return cudaSuccess;
-    cudaError_t e = reserve(n - 1);
-    if (e == cudaSuccess && n > 1) e = Api::record(forked, q);
+    std::vector<size_t> aside, on_q;
+    for (size_t k = 0; k < n; ++k) (alone(k) ? on_q : aside).push_back(k);
+    if (on_q.empty()) {
+      on_q.push_back(aside.back());
+      aside.pop_back();
+    }
+    cudaError_t e = reserve(aside.size());
+    if (e == cudaSuccess && !aside.empty()) e = Api::record(forked, q);
     size_t begun = 0;
-    for (size_t k = 0; k + 1 < n && e == cudaSuccess; ++k) {
+    for (size_t k = 0; k < aside.size() && e == cudaSuccess; ++k) {
       if ((e = Api::wait(side[k].stream, forked)) != cudaSuccess) break;
       ++begun;
-      e = f(k, side[k].stream);
+      e = f(aside[k], side[k].stream);
     }
-    if (e == cudaSuccess) e = f(n - 1, q);
+    for (size_t k = 0; k < on_q.size() && e == cudaSuccess; ++k) e = f(on_q[k], q);
     // every stream begun is joined, also after an error
     for (size_t k = 0; k < begun; ++k) {
       cudaError_t j = Api::record(side[k].joined, side[k].stream);

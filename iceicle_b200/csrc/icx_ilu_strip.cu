@@ -532,64 +532,81 @@ __global__ void strip_fill_kernel(long long n, double* ex) {
     ex[i] = v;
 }
 
+constexpr int kStripSmem = 225 * 1024, kStripCluster = 8;
+
+// a launch by clusters of strips that hand their rows over in shared memory: so many inboxes (a row of the widest
+// grid each) beside the ring; side by side with other applies no more than two chunks, so that several CTAs share an
+// SM. depth < 2: the inboxes leave no room
 template <int BS, class TA>
-cudaError_t launch_strips(const IluStripPlan& p, const StripArgs<TA>& args, bool side_by_side, cudaStream_t s) {
+struct StripClusters {
   using K = StripCfg<BS, TA>;
-  constexpr auto kern = ilu_apply_strip_kernel<BS, TA>;
-  constexpr int kSmem = 225 * 1024, kCluster = 8;
-  int dev = 0, nsm = 0;
-  cudaError_t e = cudaGetDevice(&dev);
-  if (e == cudaSuccess) e = cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
-  // the limit is a property of the kernel, shared by all threads: always the same value
-  if (e == cudaSuccess) e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmem);
-  if (e != cudaSuccess) return e;
-  StripArgs<TA> a = args;
-  // clusters of strips that hand their rows over in shared memory, where the inbox (a row of the widest grid)
-  // leaves room for two chunks; side by side with other applies no more than two, so that several CTAs share an SM
-  a.inbox = p.max_nx * BS;
-  const long long inbox = (long long)a.inbox * 8;
-  const auto fit = [&](int inboxes) { return (kSmem - K::VD * K::VB - inboxes * inbox) / K::CHUNK; };
-  if (fit(1) >= 2) {
-    cudaLaunchConfig_t cfg = {};
-    cfg.blockDim = dim3(K::NT);
-    cfg.stream = s;
-    cudaLaunchAttribute attr[2];
+  cudaLaunchConfig_t cfg = {};
+  cudaLaunchAttribute attr[2];
+  int depth = 0, resident = 0;  // chunks of the ring, clusters that run at the same time
+  static long long fit(const IluStripPlan& p, int inboxes) {
+    return (kStripSmem - K::VD * K::VB - (long long)inboxes * p.max_nx * BS * 8) / K::CHUNK;
+  }
+  StripClusters(const IluStripPlan& p, int inboxes, bool side_by_side, cudaStream_t s) {
+    depth = (int)std::min<long long>(side_by_side ? 2 : 4, fit(p, inboxes));
+    if (depth < 2) return;
     attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = kStripCluster;
     attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
     attr[1].id = cudaLaunchAttributeCooperative;
     attr[1].val.cooperative = 1;
     cfg.attrs = attr;
-    cfg.gridDim = dim3((p.nstrips + kCluster - 1) / kCluster * kCluster);
-    attr[0].val.clusterDim.x = a.cluster = kCluster;
-    int clusters = 0;
-    const auto size = [&](int inboxes) {
-      a.depth = (int)std::min<long long>(side_by_side ? 2 : 4, fit(inboxes));
-      cfg.dynamicSmemBytes = (size_t)a.depth * K::CHUNK + K::VD * K::VB + inboxes * inbox;
-      cfg.numAttrs = 1;
-      if (cudaOccupancyMaxActiveClusters(&clusters, kern, &cfg) != cudaSuccess) {
-        (void)cudaGetLastError();
-        clusters = 0;
-      }
-    };
-    // one cooperative launch for both sweeps (saves a launch and the tickets) where their inboxes leave the ring three
-    // chunks, or as many as one inbox does, and the whole grid is resident
-    if (!side_by_side && fit(2) >= std::min<long long>(3, fit(1))) {
-      size(2);
-      if ((long long)clusters * kCluster >= cfg.gridDim.x) {
-        cfg.numAttrs = 2;
-        a.sweep = 0;
-        return cudaLaunchKernelEx(&cfg, kern, a);
-      }
-    }
-    size(1);
-    if (clusters > 0) {
-      for (a.sweep = 1; a.sweep <= 2; ++a.sweep)
-        if ((e = cudaLaunchKernelEx(&cfg, kern, a)) != cudaSuccess) return e;
-      return cudaSuccess;
+    cfg.numAttrs = 1;
+    cfg.blockDim = dim3(K::NT);
+    cfg.gridDim = dim3((p.nstrips + kStripCluster - 1) / kStripCluster * kStripCluster);
+    cfg.dynamicSmemBytes = (size_t)depth * K::CHUNK + K::VD * K::VB + (size_t)inboxes * p.max_nx * BS * 8;
+    cfg.stream = s;
+    if (cudaOccupancyMaxActiveClusters(&resident, ilu_apply_strip_kernel<BS, TA>, &cfg) != cudaSuccess) {
+      (void)cudaGetLastError();
+      resident = 0;
     }
   }
+  StripClusters(const StripClusters&) = delete;
+};
+
+// the kernel's dynamic shared memory limit is its own, shared by all threads: always the same value
+template <int BS, class TA>
+cudaError_t strip_limit() {
+  return cudaFuncSetAttribute(ilu_apply_strip_kernel<BS, TA>, cudaFuncAttributeMaxDynamicSharedMemorySize, kStripSmem);
+}
+
+template <int BS, class TA>
+cudaError_t launch_strips(const IluStripPlan& p, const StripArgs<TA>& args, bool side_by_side, cudaStream_t s) {
+  using K = StripCfg<BS, TA>;
+  using C = StripClusters<BS, TA>;
+  constexpr auto kern = ilu_apply_strip_kernel<BS, TA>;
+  int dev = 0, nsm = 0;
+  cudaError_t e = cudaGetDevice(&dev);
+  if (e == cudaSuccess) e = cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
+  if (e == cudaSuccess) e = strip_limit<BS, TA>();
+  if (e != cudaSuccess) return e;
+  StripArgs<TA> a = args;
+  a.inbox = p.max_nx * BS;
+  a.cluster = kStripCluster;
+  // one cooperative launch for both sweeps (saves a launch and the tickets) where their inboxes leave the ring three
+  // chunks, or as many as one inbox does, and the whole grid is resident
+  if (!side_by_side && C::fit(p, 2) >= 2 && C::fit(p, 2) >= std::min<long long>(3, C::fit(p, 1))) {
+    C both(p, 2, false, s);
+    if ((long long)both.resident * kStripCluster >= both.cfg.gridDim.x) {
+      both.cfg.numAttrs = 2;
+      a.depth = both.depth;
+      a.sweep = 0;
+      return cudaLaunchKernelEx(&both.cfg, kern, a);
+    }
+  }
+  C each(p, 1, side_by_side, s);
+  if (each.resident > 0) {
+    a.depth = each.depth;
+    for (a.sweep = 1; a.sweep <= 2; ++a.sweep)
+      if ((e = cudaLaunchKernelEx(&each.cfg, kern, a)) != cudaSuccess) return e;
+    return cudaSuccess;
+  }
   // rows too wide for an inbox: every hand-over through L2
-  a.depth = (int)std::min<long long>(K::DMAX, (kSmem - K::VD * K::VB) / K::CHUNK);
+  a.depth = (int)std::min<long long>(K::DMAX, (kStripSmem - K::VD * K::VB) / K::CHUNK);
   a.cluster = 1;
   a.sweep = 0;
   const size_t smem = (size_t)a.depth * K::CHUNK + K::VD * K::VB;
@@ -643,6 +660,16 @@ long long ilu_strip_bytes(int bs, int nx, int nr, bool f32) {
   ICX_STRIP_SIZES(ICX_STRIP_CASE)
 #undef ICX_STRIP_CASE
   return 0;
+}
+
+bool la_ilu_strips_resident(int bs, const IluStripPlan& p, bool f32) {
+#define ICX_STRIP_CASE(B)                                                                                           \
+  if (bs == B)                                                                                                      \
+    return f32 ? strip_limit<B, float>() != cudaSuccess || StripClusters<B, float>(p, 1, true, 0).resident == 0     \
+               : strip_limit<B, double>() != cudaSuccess || StripClusters<B, double>(p, 1, true, 0).resident == 0;
+  ICX_STRIP_SIZES(ICX_STRIP_CASE)
+#undef ICX_STRIP_CASE
+  return true;
 }
 
 cudaError_t la_ilu_strip_reset(const IluStripPlan& p, cudaStream_t s) {

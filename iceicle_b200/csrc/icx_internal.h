@@ -252,6 +252,8 @@ icx_status solver_take_pc_err(icx_ctx* c, int* err);
 // flag, whether the preconditioner apply can be captured in a graph, and the
 // reference's line searches (1 Wolfe, 2 Corrigan, else the full step)
 icx_status solver_group_ready(icx_ctx* c, int precision, int pc_sweeps, int ilu_tile, bool graphs, bool side_by_side);
+// whether an apply of the preconditioner is a launch whose CTAs wait on one another and fill the GPU
+bool solver_pc_whole_gpu(icx_ctx* c, int kind, bool mixed);
 cudaError_t solver_linearise(icx_ctx* c, const double* u, double* res, int precision, cudaStream_t s);
 cudaError_t solver_build_pc(icx_ctx* c, int kind, bool mixed, cudaStream_t s);
 cudaError_t solver_operator(icx_ctx* c, bool mixed, const double* x, double* y, cudaStream_t s);

@@ -82,6 +82,8 @@ cudaError_t la_ilu_strip_pack(int bs, const IluStripPlan& p, const double* LU, c
                               cudaStream_t s);
 cudaError_t la_ilu_strip_pack_f32(int bs, const IluStripPlan& p, const double* LU, const double* Uinv, float* pk,
                                   cudaStream_t s);
+// whether a side-by-side apply is a launch that has to be resident as a whole (rows too wide for the clusters)
+bool la_ilu_strips_resident(int bs, const IluStripPlan& p, bool f32);
 // y = (LU)^-1 x; f = n doubles of scratch; *err = 1 if a wait ran out; side_by_side: applies of other plans run
 // at the same time on other streams
 cudaError_t la_ilu_apply_strips(int bs, const IluStripPlan& p, const double* pk, const double* x, double* y, double* f,

@@ -285,10 +285,12 @@ cudaError_t put_per_part(icx_pset* S, const std::vector<double>& v, double* dst,
 // their own and their parts of the set's vectors do not overlap; their launches
 // are bound by latency (the block-ILU(0) apply above all) and leave most of the
 // GPU to one another: set of 16 problems, orders 1 to 4, 603 ms in turn, 351 ms
-// side by side
+// side by side. Groups whose piece fills the GPU with CTAs that wait on one
+// another (`alone`) run in turn on q: no two of them share the SMs
 cudaError_t all_groups(icx_pset* S, cudaStream_t q,
-                       const std::function<cudaError_t(icx_ctx*, long long, cudaStream_t)>& f) {
-  return S->forks.run(S->groups.size(), q,
+                       const std::function<cudaError_t(icx_ctx*, long long, cudaStream_t)>& f,
+                       const std::function<bool(icx_ctx*)>& alone = [](icx_ctx*) { return false; }) {
+  return S->forks.run(S->groups.size(), q, [&](size_t g) { return alone(S->groups[g]); },
                       [&](size_t g, cudaStream_t t) { return f(S->groups[g], S->group_off[g], t); });
 }
 
@@ -324,6 +326,7 @@ icx_status pset_gmres(icx_pset* S, int pc, bool mixed, int m, int maxit, double 
     K[p].y.assign(m, 0.0);
   }
   PCK(cudaMemcpyAsync(S->r, b, sizeof(double) * N, cudaMemcpyDeviceToDevice, s));
+  const auto alone = [&](icx_ctx* g) { return icx::solver_pc_whole_gpu(g, pc, mixed); };
   // graphs of the Arnoldi steps, valid while the key holds
   bool graphable = true;
   unsigned long long key = 1469598103934665603ull;
@@ -367,7 +370,7 @@ icx_status pset_gmres(icx_pset* S, int pc, bool mixed, int m, int maxit, double 
           cudaError_t ee = pc ? icx::solver_apply_pc(g, pc, mixed, vj + off, S->z + off, t) : cudaSuccess;
           if (ee == cudaSuccess) ee = icx::solver_operator(g, mixed, (pc ? S->z : vj) + off, vj1 + off, t);
           return ee;
-        });
+        }, alone);
         for (int pass = 0; pass < passes && e == cudaSuccess; ++pass) {
           double* slot = S->dots + (size_t)pass * P * ld;
           e = seg_dots(S, S->V, N, j + 1, vj1, slot, ld, q);
@@ -470,7 +473,7 @@ icx_status pset_gmres(icx_pset* S, int pc, bool mixed, int m, int maxit, double 
     if (pc) {
       PCK(all_groups(S, s, [&](icx_ctx* g, long long off, cudaStream_t t) {
         return icx::solver_apply_pc(g, pc, mixed, S->w + off, S->z + off, t);
-      }));
+      }, alone));
       PCK(icx::la_axpby(N, 1.0, S->z, 1.0, x, s));
     } else {
       PCK(icx::la_axpby(N, 1.0, S->w, 1.0, x, s));

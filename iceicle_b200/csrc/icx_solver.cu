@@ -1324,6 +1324,15 @@ cudaError_t solver_apply_pc(icx_ctx* c, int kind, bool mixed, const double* x, d
   return apply_pc(c, kind, mixed, x, z, s);
 }
 
+bool solver_pc_whole_gpu(icx_ctx* c, int kind, bool mixed) {
+  icx_solver_work* w = c->sw;
+  const int pi = mixed ? 1 : 0;
+  if (kind != 2 || !w) return false;
+  if (w->tp.tile) return !(w->tp.group_ok && ilu_schedule(c->dm.tile, pi, true) >= 3);
+  if (w->rows_ok && w->schedule == 2) return true;
+  return !(w->sp_ok[pi] && strip_shape(c, mixed)) || la_ilu_strips_resident(w->bs, w->sp[pi], mixed);
+}
+
 cudaError_t solver_pack_strips(icx_ctx* c, bool mixed, cudaStream_t s) { return pack_strips(c, mixed, s); }
 
 const float* solver_vals32(icx_ctx* c) { return c->sw ? c->sw->vals32 : nullptr; }

@@ -58,6 +58,7 @@ static int bad = 0;
 
 int main() {
   const cudaStream_t q = nullptr;
+  const auto none = [](size_t) { return false; };
   // each creation in turn fails; the call after it has all it needs
   for (int n = 1; n <= 4; ++n)
     for (int k = 1; k <= 2 * n; ++k) {
@@ -70,30 +71,48 @@ int main() {
         CHECK(used.insert(t).second);
         return cudaSuccess;
       };
-      const cudaError_t e = forks.run(n, q, f);
+      const cudaError_t e = forks.run(n, q, none, f);
       CHECK((e == cudaSuccess) == (k > calls));
       CHECK(e == cudaSuccess || used.empty());
       fail_at = 0;
       used.clear();
       after.clear();
-      CHECK(forks.run(n, q, f) == cudaSuccess);
+      CHECK(forks.run(n, q, none, f) == cudaSuccess);
       CHECK((int)used.size() == n && used.count(q));
       for (cudaStream_t t : used)  // forked from q and joined to it
         if (t != q) CHECK(after[t].count(q) && after[q].count(t));
       forks.release();
       CHECK(live == 0);
     }
+  // pieces that run alone: on q, in their order; the others have a side stream each
+  for (unsigned mask = 1; mask < 32; ++mask) {
+    icx::Forks<Fake> forks;
+    after.clear();
+    size_t last = 0;
+    std::set<cudaStream_t> used;
+    CHECK(forks.run(5, q, [&](size_t k) { return (mask >> k & 1) != 0; }, [&](size_t k, cudaStream_t t) {
+      if (mask >> k & 1) {
+        CHECK(t == q && last <= k);
+        last = k;
+      } else {
+        CHECK(t != q && used.insert(t).second);
+      }
+      return cudaSuccess;
+    }) == cudaSuccess);
+    for (cudaStream_t t : used) CHECK(after[t].count(q) && after[q].count(t));
+    forks.release();
+  }
   // a piece that fails: the streams begun are joined all the same
   icx::Forks<Fake> forks;
   after.clear();
   std::set<cudaStream_t> used;
-  CHECK(forks.run(4, q, [&](size_t k, cudaStream_t t) {
+  CHECK(forks.run(4, q, none, [&](size_t k, cudaStream_t t) {
     used.insert(t);
     return k == 1 ? cudaErrorLaunchFailure : cudaSuccess;
   }) == cudaErrorLaunchFailure);
   CHECK(used.size() == 2);
   for (cudaStream_t t : used) CHECK(after[q].count(t));
-  CHECK(forks.run(0, q, [&](size_t, cudaStream_t) { return cudaErrorUnknown; }) == cudaSuccess);
+  CHECK(forks.run(0, q, none, [&](size_t, cudaStream_t) { return cudaErrorUnknown; }) == cudaSuccess);
   forks.release();
   if (!bad) std::printf("ok\n");
   return bad;
