@@ -399,6 +399,12 @@ icx_status ensure_ilu_plan(icx_ctx* c) {
       return set_err(c, ICX_ERR_CUDA, std::string("tiled ILU plan: ") + cudaGetErrorString(e));
     }
   }
+  // the copies are on the legacy stream, from pageable memory: a kernel on a stream that does not wait for that one
+  // (a caller's, a set's side streams) must find them done
+  if (const cudaError_t e = cudaStreamSynchronize(0); e != cudaSuccess) {
+    free_tile_plan(tp);
+    return set_err(c, ICX_ERR_CUDA, std::string("tiled ILU plan: ") + cudaGetErrorString(e));
+  }
   tp.tile = st;
   tp.gen = c->ilu_plan_gen;
   w->tp = std::move(tp);
