@@ -804,7 +804,18 @@ cudaError_t la_mdot32(LinalgWork& w, long long n, const float* V, long long ld, 
 cudaError_t la_mdot_alloc(LinalgWork& w) {
   if (w.partial) return cudaSuccess;
   cudaError_t e = cudaMalloc((void**)&w.partial, sizeof(double) * (64 * kMdotBlocks + 1));
-  if (e == cudaSuccess) e = cudaMemset(w.ticket(), 0, sizeof(double));
+  if (e != cudaSuccess) {
+    w.partial = nullptr;
+    return e;
+  }
+  // the ticket is zero before any stream, also one that does not wait for the legacy one, uses it; without that
+  // there are no buffers
+  e = cudaMemset(w.ticket(), 0, sizeof(double));
+  if (e == cudaSuccess) e = cudaStreamSynchronize(0);
+  if (e != cudaSuccess) {
+    cudaFree(w.partial);
+    w.partial = nullptr;
+  }
   return e;
 }
 
