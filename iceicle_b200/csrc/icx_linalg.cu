@@ -574,6 +574,12 @@ __global__ void __launch_bounds__(FacCfg<BS>::THREADS) ilu_level_kernel(int E, i
           else if (p.x < BS && p.y < BS) LU[(size_t)ej * B2 + p.x * BS + p.y] -= acc[m];
         }
       }
+      if (K::NBUF == 6 && jc < e && n + 1 < nl) {  // this may be the next neighbour's A_ek, staged as it was before
+        cp_async_wait<0>();
+        __syncthreads();
+        double* Xn = sh + (size_t)(3 * ((n + 1) & 1)) * K::B2P;
+        for (int t = tid; t < B2; t += blockDim.x) Xn[t / BS * LD + t % BS] = LU[(size_t)(kl + 1) * B2 + t];
+      }
     }
     // buffers of this neighbour are free
     if (n + (K::NBUF == 6 ? 2 : 1) < nl) {

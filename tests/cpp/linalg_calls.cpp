@@ -46,4 +46,16 @@ int strip_apply(int bs, int nstrips, int max_steps, int max_nx, void* strips, do
                                               0));
 }
 
+int ilu_factor(int E, int bs, int nnzb, int* rowptr, int* colidx, const int* order, const int* lvl_off, int n_levels,
+               double* LU, double* Uinv, int* flag) {
+  icx::DeviceMesh dm{};
+  dm.E = E;
+  dm.nb = bs;
+  dm.neq = 1;
+  dm.nnzb = nnzb;
+  dm.bsr_rowptr = rowptr;
+  dm.bsr_colidx = colidx;
+  return (int)icx::la_ilu_factor(dm, order, std::vector<int>(lvl_off, lvl_off + n_levels + 1), LU, Uinv, flag, 0);
+}
+
 }  // extern "C"
