@@ -185,11 +185,11 @@ icx_status ensure_explicit(icx_ctx* c) {
   w->n = n;
   w->E = dm.E;
   w->nb = dm.nb;
-  XCK(cudaMalloc((void**)&w->minv, sizeof(double) * (size_t)dm.E * dm.nb * dm.nb));
-  XCK(cudaMalloc((void**)&w->singular, sizeof(int) * dm.E));
+  XCK(icx::ctx_malloc(c, (void**)&w->minv, sizeof(double) * (size_t)dm.E * dm.nb * dm.nb));
+  XCK(icx::ctx_malloc(c, (void**)&w->singular, sizeof(int) * dm.E));
   double** vecs[] = {&w->r, &w->d1, &w->d2, &w->d3, &w->uold};
-  for (double** p : vecs) XCK(cudaMalloc((void**)p, sizeof(double) * n));
-  XCK(cudaMalloc((void**)&w->lam, sizeof(unsigned long long)));
+  for (double** p : vecs) XCK(icx::ctx_malloc(c, (void**)p, sizeof(double) * n));
+  XCK(icx::ctx_malloc(c, (void**)&w->lam, sizeof(unsigned long long)));
   return ICX_OK;
 }
 

@@ -243,6 +243,11 @@ const float* solver_vals32(icx_ctx* c);
 // solver_prepare_pc with kind 2), and the apply's error flag (read, then
 // cleared with the completion counters when set)
 cudaError_t solver_apply_ilu_flow(icx_ctx* c, bool mixed, const double* x, double* z, cudaStream_t s);
+// device memory for a context's work; where it is short, what the context can do without (the strips' packed copies of
+// the factors) is given back first
+cudaError_t ctx_malloc(icx_ctx* c, void** p, size_t bytes);
+// frees the packed copies (and the graphs that hold their addresses); false if there were none
+bool solver_give_back(icx_ctx* c);
 // the whole-grid apply's packed factors of one precision, from the factors in place, at the context's tile choice
 cudaError_t solver_pack_strips(icx_ctx* c, bool mixed, cudaStream_t s);
 icx_status solver_take_pc_err(icx_ctx* c, int* err);

@@ -238,9 +238,19 @@ icx_status ensure_buffers(icx_pset* S, int m) {
   if (S->m >= m) return ICX_OK;
   free_buffers(S);
   const size_t n = (size_t)S->N, ld = (size_t)m + 2, P = (size_t)S->n_parts;
-  PCK(cudaMalloc((void**)&S->V, sizeof(double) * (m + 1) * n));
+  // the large ones: where memory is short, what the groups can do without is given back first
+  const auto get = [&](double** p, size_t bytes) {
+    cudaError_t e = cudaMalloc((void**)p, bytes);
+    for (size_t g = 0; g < S->groups.size() && e == cudaErrorMemoryAllocation; ++g) {
+      (void)cudaGetLastError();
+      if (icx::solver_give_back(S->groups[g])) e = cudaMalloc((void**)p, bytes);
+    }
+    if (e != cudaSuccess) *p = nullptr;
+    return e;
+  };
+  PCK(get(&S->V, sizeof(double) * (m + 1) * n));
   double** vecs[] = {&S->w, &S->z, &S->r, &S->res, &S->du, &S->ut, &S->rt};
-  for (double** p : vecs) PCK(cudaMalloc((void**)p, sizeof(double) * n));
+  for (double** p : vecs) PCK(get(p, sizeof(double) * n));
   PCK(cudaMalloc((void**)&S->partial, sizeof(double) * (size_t)S->n_chunks * ld));
   PCK(cudaMalloc((void**)&S->dots, sizeof(double) * 3 * P * ld));
   PCK(cudaMalloc((void**)&S->coef, sizeof(double) * P * ld));

@@ -14,6 +14,7 @@
 #include <cstdint>
 #include <cstring>
 #include <functional>
+#include <initializer_list>
 #include <map>
 #include <vector>
 
@@ -248,12 +249,24 @@ icx_status build_strip_plan(icx_ctx* c) {
     }
     e0 += nx * ny;
   }
+  // without memory for the strips the data-flow apply stays
   double* ex = nullptr;
-  CK(cudaMalloc((void**)&ex, sizeof(double) * nex));
+  unsigned long long* ticket = nullptr;
+  icx::IluStrip* ds[2] = {nullptr, nullptr};
+  if (cudaMalloc((void**)&ex, sizeof(double) * nex) != cudaSuccess ||
+      cudaMalloc((void**)&ticket, sizeof(unsigned long long)) != cudaSuccess ||
+      cudaMalloc((void**)&ds[0], sizeof(icx::IluStrip) * strips.size()) != cudaSuccess ||
+      cudaMalloc((void**)&ds[1], sizeof(icx::IluStrip) * strips.size()) != cudaSuccess) {
+    (void)cudaGetLastError();
+    for (void* p : {(void*)ex, (void*)ticket, (void*)ds[0], (void*)ds[1]})
+      if (p) cudaFree(p);
+    return ICX_OK;
+  }
   w->sp[0].ex = w->sp[1].ex = ex;
-  CK(cudaMalloc((void**)&w->sp[0].ticket, sizeof(unsigned long long)));
-  CK(cudaMemset(w->sp[0].ticket, 0, sizeof(unsigned long long)));
-  w->sp[1].ticket = w->sp[0].ticket;
+  w->sp[0].ticket = w->sp[1].ticket = ticket;
+  w->sp[0].strips = ds[0];
+  w->sp[1].strips = ds[1];
+  CK(cudaMemset(ticket, 0, sizeof(unsigned long long)));
   for (int pi = 0; pi < 2; ++pi) {
     icx::IluStripPlan& sp = w->sp[pi];
     sp.nex = nex;
@@ -263,7 +276,6 @@ icx_status build_strip_plan(icx_ctx* c) {
       sp.max_steps = std::max(sp.max_steps, s.nx + s.nr - 1);
       sp.max_nx = std::max(sp.max_nx, s.nx);
     }
-    CK(cudaMalloc((void**)&sp.strips, sizeof(icx::IluStrip) * strips.size()));
     CK(cudaMemcpy(sp.strips, strips.data(), sizeof(icx::IluStrip) * strips.size(), cudaMemcpyHostToDevice));
   }
   CK(icx::la_ilu_strip_reset(w->sp[0], 0));
@@ -441,26 +453,39 @@ double dev_norm(icx_ctx* c, const double* x, cudaStream_t s) {
   return std::sqrt(h);
 }
 
+// all of the buffers or none
+icx_status alloc_all(icx_ctx* c, std::initializer_list<std::pair<void**, size_t>> buffers) {
+  for (const auto& b : buffers) {
+    const cudaError_t e = icx::ctx_malloc(c, b.first, b.second);
+    if (e == cudaSuccess) continue;
+    for (const auto& q : buffers) {
+      if (q.first == b.first) break;
+      cudaFree(*q.first);
+      *q.first = nullptr;
+    }
+    return set_err(c, ICX_ERR_CUDA, std::string("solver buffers: ") + cudaGetErrorString(e));
+  }
+  return ICX_OK;
+}
+
 // FP32 copies of the Jacobian and preconditioner (mixed precision), allocated on first use
 icx_status ensure_mixed(icx_ctx* c) {
   icx_solver_work* w = c->sw;
   if (w->vals32) return ICX_OK;
   size_t nv = (size_t)w->nnzb * w->bs * w->bs;
-  CK(cudaMalloc((void**)&w->vals32, sizeof(float) * nv));
-  CK(cudaMalloc((void**)&w->pc32, sizeof(float) * nv));
-  CK(cudaMalloc((void**)&w->uinv32, sizeof(float) * (size_t)c->dm.E * w->bs * w->bs));
-  CK(cudaMalloc((void**)&w->V32, sizeof(float) * (size_t)(w->m + 1) * w->n));
-  CK(cudaMalloc((void**)&w->vt, sizeof(double) * w->n));
-  return ICX_OK;
+  return alloc_all(c, {{(void**)&w->vals32, sizeof(float) * nv},
+                       {(void**)&w->pc32, sizeof(float) * nv},
+                       {(void**)&w->uinv32, sizeof(float) * (size_t)c->dm.E * w->bs * w->bs},
+                       {(void**)&w->V32, sizeof(float) * (size_t)(w->m + 1) * w->n},
+                       {(void**)&w->vt, sizeof(double) * w->n}});
 }
 
 icx_status ensure_bf16(icx_ctx* c) {
   icx_solver_work* w = c->sw;
   if (w->pc16) return ICX_OK;
   size_t nv = (size_t)w->nnzb * w->bs * w->bs;
-  CK(cudaMalloc((void**)&w->pc16, sizeof(__nv_bfloat16) * nv));
-  CK(cudaMalloc((void**)&w->uinv16, sizeof(__nv_bfloat16) * (size_t)c->dm.E * w->bs * w->bs));
-  return ICX_OK;
+  return alloc_all(c, {{(void**)&w->pc16, sizeof(__nv_bfloat16) * nv},
+                       {(void**)&w->uinv16, sizeof(__nv_bfloat16) * (size_t)c->dm.E * w->bs * w->bs}});
 }
 
 cudaError_t diag_apply(icx_ctx* c, bool mixed, const double* D, const float* D32, const double* x, double* z,
@@ -746,7 +771,8 @@ icx_status gmres(icx_ctx* c, int pc, bool mixed, int m, int maxit, double rtol, 
                         (long long)(uintptr_t)dm.bsr_colidx, (long long)(uintptr_t)dm.bsr_diag,
                         (long long)(uintptr_t)w->order, (long long)w->tp.tile, (long long)(uintptr_t)w->tp.order,
                         (long long)w->fd_on, (long long)(uintptr_t)w->fd_u, (long long)(uintptr_t)w->fd_r,
-                        (long long)w->bf16, (long long)w->cgs_passes, (long long)w->sp_ok[pi]})
+                        (long long)w->bf16, (long long)w->cgs_passes,
+                        (long long)(uintptr_t)(w->sp_ok[pi] ? w->spk[pi] : nullptr)})
       key = (key ^ (unsigned long long)v) * 1099511628211ull;
     kb.graphs = &w->graphs;
     kb.graph_key = key | 1;
@@ -1339,6 +1365,28 @@ bool solver_pc_whole_gpu(icx_ctx* c, int kind, bool mixed) {
   return !(w->sp_ok[pi] && strip_shape(c, mixed)) || la_ilu_strips_resident(w->bs, w->sp[pi], mixed);
 }
 
+bool solver_give_back(icx_ctx* c) {
+  icx_solver_work* w = c ? c->sw : nullptr;
+  if (!w || !(w->spk[0] || w->spk[1])) return false;
+  w->graphs.release();
+  for (int pi = 0; pi < 2; ++pi) {
+    if (w->spk[pi]) cudaFree(w->spk[pi]);  // waits for the applies that read it
+    w->spk[pi] = nullptr;
+    w->sp_ok[pi] = false;
+  }
+  return true;
+}
+
+cudaError_t ctx_malloc(icx_ctx* c, void** p, size_t bytes) {
+  cudaError_t e = cudaMalloc(p, bytes);
+  if (e == cudaErrorMemoryAllocation) {
+    (void)cudaGetLastError();
+    if (solver_give_back(c) && (e = cudaMalloc(p, bytes)) != cudaSuccess) (void)cudaGetLastError();
+  }
+  if (e != cudaSuccess) *p = nullptr;
+  return e;
+}
+
 cudaError_t solver_pack_strips(icx_ctx* c, bool mixed, cudaStream_t s) { return pack_strips(c, mixed, s); }
 
 const float* solver_vals32(icx_ctx* c) { return c->sw ? c->sw->vals32 : nullptr; }
@@ -1402,7 +1450,8 @@ unsigned long long solver_graph_key(icx_ctx* c, int pc, bool mixed) {
                       (long long)t.flow_ctas[pi], (long long)t.flow_sched[pi], (long long)(uintptr_t)dm.bsr_rowptr,
                       (long long)(uintptr_t)dm.bsr_colidx, (long long)(uintptr_t)dm.bsr_diag,
                       (long long)(uintptr_t)w->order, (long long)w->tp.tile, (long long)(uintptr_t)w->tp.order,
-                      (long long)(uintptr_t)w->vals, (long long)(uintptr_t)w->pc, (long long)w->sp_ok[pi]})
+                      (long long)(uintptr_t)w->vals, (long long)(uintptr_t)w->pc,
+                      (long long)(uintptr_t)(w->sp_ok[pi] ? w->spk[pi] : nullptr)})
     key = (key ^ (unsigned long long)v) * 1099511628211ull;
   return key;
 }

@@ -81,8 +81,8 @@ struct Scratch {
       if (e) cudaEventDestroy(e);
   }
   template <class T>
-  cudaError_t alloc(T** p, size_t bytes) {
-    cudaError_t e = cudaMalloc((void**)p, bytes);
+  cudaError_t alloc(icx_ctx* c, T** p, size_t bytes) {
+    cudaError_t e = icx::ctx_malloc(c, (void**)p, bytes);
     if (e == cudaSuccess) ptrs.push_back(*p);
     return e;
   }
@@ -97,8 +97,8 @@ struct Tuner {
   int timed = 0, rejected = 0;
 
   icx_status init() {
-    TCK(sc.alloc(&flush, FLUSH_BYTES));
-    TCK(sc.alloc(&diff, sizeof(unsigned long long)));
+    TCK(sc.alloc(c, &flush, FLUSH_BYTES));
+    TCK(sc.alloc(c, &diff, sizeof(unsigned long long)));
     TCK(cudaEventCreate(&sc.ev[0]));
     TCK(cudaEventCreate(&sc.ev[1]));
     return ICX_OK;
@@ -139,8 +139,8 @@ struct Tuner {
     icx::DeviceMesh& dm = c->dm;
     const long long n = (long long)dm.E * dm.nb * dm.neq;
     double *r0 = nullptr, *r1 = nullptr;
-    TCK(sc.alloc(&r0, sizeof(double) * n));
-    TCK(sc.alloc(&r1, sizeof(double) * n));
+    TCK(sc.alloc(c, &r0, sizeof(double) * n));
+    TCK(sc.alloc(c, &r1, sizeof(double) * n));
     const TileChoice keep = dm.tile;
     dm.tile.face_minb = 0;
     dm.tile.vol_threads = dm.tile.vol_minb = 0;
@@ -190,11 +190,11 @@ struct Tuner {
     const int bs = dm.nb * dm.neq;
     const long long n = (long long)dm.E * bs;
     double *vals = nullptr, *res = nullptr, *x = nullptr, *z0 = nullptr, *z1 = nullptr;
-    TCK(sc.alloc(&vals, sizeof(double) * (size_t)dm.nnzb * bs * bs));
-    TCK(sc.alloc(&res, sizeof(double) * n));
-    TCK(sc.alloc(&x, sizeof(double) * n));
-    TCK(sc.alloc(&z0, sizeof(double) * n));
-    TCK(sc.alloc(&z1, sizeof(double) * n));
+    TCK(sc.alloc(c, &vals, sizeof(double) * (size_t)dm.nnzb * bs * bs));
+    TCK(sc.alloc(c, &res, sizeof(double) * n));
+    TCK(sc.alloc(c, &x, sizeof(double) * n));
+    TCK(sc.alloc(c, &z0, sizeof(double) * n));
+    TCK(sc.alloc(c, &z1, sizeof(double) * n));
     TCK(icx::launch_jacobian_fd(dm, c->phys, u, res, vals, std::sqrt(DBL_EPSILON), s));
     fill_hash_kernel<<<592, 256, 0, s>>>(x, n);
     TCK(cudaGetLastError());
