@@ -574,12 +574,15 @@ cudaError_t tile_launch(const IluGroupArgs<TS>& args, int nlev_max, cudaStream_t
     if (args.plan.ngroups > 2 * c * sms) return cudaErrorNotSupported;
     kern = (const void*)ilu_apply_tile_rows_kernel<BS, TS>;
     nt = TileRowCfg<BS>::NT + 32;
-  } else if (sizeof(TS) == 8 || c == 1) {
+  } else {
     kern = (const void*)ilu_apply_tile_kernel<BS, TS, 8, 1>;
     nt = 8 * 32 + 32;
-  } else {
-    kern = (const void*)ilu_apply_tile_kernel<BS, TS, 4, sizeof(TS) == 8 ? 1 : 3>;
-    nt = 4 * 32 + 32;
+    if constexpr (sizeof(TS) < 8) {
+      if (c > 1) {
+        kern = (const void*)ilu_apply_tile_kernel<BS, TS, 4, 3>;
+        nt = 4 * 32 + 32;
+      }
+    }
   }
   const size_t smem = (size_t)nslot * K::SLOT + tile_fixed_smem<BS, TS>(gmax);
   // the limit is a property of the kernel, shared by all threads: always the same value (tile_slots leaves 2048 bytes

@@ -584,8 +584,7 @@ __global__ void __launch_bounds__((JacCfg<PDE, P, G, T>::THREADS), (JacCfg<PDE, 
   }
 }
 
-// ------------------------------------------------------------------ SpMV
-// y = J x; one warp per block row, lanes over the rows of the block
+// the element kernel of one (PDE, order, geometry order), with the DDG flux's second derivatives or without
 template <int PDE, int P, int G, class T>
 static cudaError_t jac_pg(const DeviceMesh& dm, const PhysParams& pp, const double* u, T* vals, double eps,
                           cudaStream_t s) {
@@ -635,6 +634,8 @@ cudaError_t launch_jacobian_fd_f32(const DeviceMesh& dm, const PhysParams& pp, c
   return jac_dispatch<float>(dm, pp, u, vals, std::sqrt((double)FLT_EPSILON), s);
 }
 
+// ------------------------------------------------------------------ SpMV
+// y = J x; one warp per block row, lanes over the rows of the block
 cudaError_t launch_bsr_spmv(const DeviceMesh& dm, const double* vals, const double* x, double* y, cudaStream_t s) {
   int bs = dm.nb * dm.neq;
   RowSet rs{0, 0, -1, dm.E};
