@@ -114,7 +114,7 @@ cudaError_t ilu_apply_groups_t(const DeviceMesh& dm, const IluGroupShape& gs, co
   ICX_BLOCK_SIZES(ICX_ILUG_CASE)
 #undef ICX_ILUG_CASE
   if (!k.kern) return cudaErrorInvalidValue;
-  if (k.smem > 48 * 1024) {
+  if (k.smem + 2048 > 48 * 1024) {  // with the kernel's static shared memory above what needs no limit
     // the limit is a property of the kernel, shared by all threads: always the same value
     cudaError_t e = cudaFuncSetAttribute(k.kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_avail());
     if (e != cudaSuccess) return e;
@@ -141,7 +141,7 @@ cudaError_t la_ilu_apply_groups_bf16(const DeviceMesh& dm, const IluGroupShape& 
   ICX_BLOCK_SIZES(ICX_ILUG16_CASE)
 #undef ICX_ILUG16_CASE
   if (!k.kern) return cudaErrorNotSupported;  // the one-lane-per-row form does not fit
-  if (k.smem > 48 * 1024) {
+  if (k.smem + 2048 > 48 * 1024) {  // with the kernel's static shared memory above what needs no limit
     // the limit is a property of the kernel, shared by all threads: always the same value
     cudaError_t e = cudaFuncSetAttribute(k.kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_avail());
     if (e != cudaSuccess) return e;
