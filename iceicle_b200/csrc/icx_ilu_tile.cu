@@ -551,12 +551,34 @@ int device_attr(cudaDeviceAttr attr) {
   return v;
 }
 
+// Groups for which the forms of before are ahead: a group's table, barriers and first copies are a fixed cost that
+// few elements do not repay, and 16 x 16 blocks in FP32 on wide levels run a lane per row on 512 threads there. Both
+// sides in us, the form of before first:
+//   FP64  groups of less than 96 rows in more than two rounds over the SMs (160 x 160 elements, 2 x 2 tiles: 4 x 4
+//         blocks 59 / 80, 16 x 16 125 / 148; single 36 x 36 blocks 471 / 636; from 96 rows on 1.0 to 1.6 times
+//         ahead here), and single 4 x 4 blocks (6.0 / 6.3)
+//   FP32  single blocks (4.3 / 6.3; 64 x 64 in any number, 11.5 / 13.0) and groups of less than 8 of 36 x 36 (2 x 2
+//         tiles 8.4 / 10.5), in up to two rounds; 16 x 16 blocks in groups of more than 256 on up to a quarter of the SMs, where the lane-per-row
+//         form fits (one tile of 32 x 32: 186 / 244; 64 tiles of 24 x 24: 190 / 168)
+//   BF16  single 36 x 36 blocks (4.3 / 6.3); groups of less than 12 of 64 x 64 (2 x 2 tiles, 160 x 160: 193 / 285;
+//         4 x 4 tiles: 244 / 209)
+template <int BS, class TS>
+bool tile_behind(const IluGroupPlan& plan, int nlev_max, int sms, int optin) {
+  const int g = plan.gmax, n = plan.ngroups;
+  if (sizeof(TS) == 8) return g * BS < 16 || (g * BS < 96 && n > 2 * sms);
+  if (sizeof(TS) == 2) return g < (BS == 36 ? 2 : 12);
+  if (g < 2 && (BS == 64 || n <= 2 * sms)) return true;
+  if (BS == 36 && g < 8 && n <= 2 * sms) return true;
+  return BS == 16 && g > 256 && n <= sms / 4 && nlev_max <= kGroupLevelsSmem &&
+         group_rows_smem<float>(g, BS) + 2048 <= (size_t)optin;
+}
+
 template <int BS, class TS>
 cudaError_t tile_launch(const IluGroupArgs<TS>& args, int nlev_max, cudaStream_t s) {
   using K = TileCfg<BS, TS>;
   const int optin = device_attr(cudaDevAttrMaxSharedMemoryPerBlockOptin);
   const int sms = device_attr(cudaDevAttrMultiProcessorCount);
-  if (optin <= 0 || sms <= 0) return cudaErrorNotSupported;
+  if (optin <= 0 || sms <= 0 || tile_behind<BS, TS>(args.plan, nlev_max, sms, optin)) return cudaErrorNotSupported;
   // as many CTAs on an SM as there are groups for (FP32 up to three, the row kernel two; FP64 reaches the copy
   // rate with one) while each keeps a ring worth having: four slots, the row kernel eight, since a chunk takes
   // that many at once (16 x 16 tiles in BF16: 212 us with one CTA of 16 slots, 272 with two of 4). Eight consumer
