@@ -9,9 +9,11 @@
 // an exchange buffer in global memory: the producer stores its last row there,
 // and one warp of the consumer (the fetcher) reads that row ahead of the steps,
 // re-reading slots that still hold a sentinel and putting the sentinel back once
-// read, so that a finished apply leaves the buffer ready for the next one. A
-// strip follows its neighbour at a distance of one hand-over; after that both
-// run at the pace of the in-CTA steps.
+// read, so that a finished apply leaves the buffer ready for the next one (inside
+// a cluster the row goes straight into the consumer's shared memory). A strip
+// that is given up leaves NaN, never what y held before. A strip follows its
+// neighbour at a distance of one hand-over; after that both run at the pace of
+// the in-CTA steps.
 //
 // The factors are repacked once per factorisation in the order in which the
 // steps read them: a step's blocks of all rows are one contiguous piece, entry
@@ -24,8 +26,10 @@
 // for bit.
 //
 // Against the data-flow apply, whose every level is a trip through L2 (FP64 /
-// FP32): NS p = 2 256 x 256 1.70 -> 1.02 / 1.56 -> 0.91 ms, 128 x 128 715 -> 452
-// us; a Newton solve on 32 x 32 Burgers elements (P2) 131 -> 71 ms.
+// FP32): NS p = 2 256 x 256 1.69 -> 1.03 / 1.56 -> 0.91 ms, 128 x 128 716 -> 448
+// us; Burgers p = 2 32 x 32 139 -> 45 us (a Newton solve 132 -> 62 ms, with the
+// dot products' steps); also ahead on one row or column of 1000 elements and on
+// rows too wide for an inbox (NS p = 2 400 x 400 3.29 -> 3.00 ms).
 #include <algorithm>
 #include <vector>
 

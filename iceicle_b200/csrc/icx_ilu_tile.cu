@@ -20,13 +20,15 @@
 // LPR VEC fold inside the lane, the next ones across the row's lanes, the last
 // ones inside the lane again.
 //
-// Measured (NS, 8 x 8 tiles, BS = 36), against the forms it replaces:
+// Measured (NS, 8 x 8 tiles, BS = 36; calls on one vector in turn), against the
+// forms it replaces:
 //                              before      here    factors at 6.45 TB/s
-//   FP64   256 x 256            917 us    487 us    474 us
-//   FP64   128 x 128            242       136       118
-//   FP32   256 x 256            500       278       237
-//   FP32   128 x 128            146        71        59
-//   BF16   128 x 128 (rows)      94        49        30
+//   FP64   256 x 256            922 us    487 us    474 us
+//   FP64   128 x 128            241       136       118
+//   FP32   256 x 256            501       278       237
+//   FP32   128 x 128            146        72        59
+//   BF16   128 x 128 (rows)      95        47        30
+// (FP64 256 x 256 with other inputs from call to call 924 and 515.)
 // Below some 148 tiles the levels' own latency is left (32 x 32: 54, 41 and 33 us
 // for 30 levels; 177, 54 and 58 before).
 //

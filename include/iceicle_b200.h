@@ -628,7 +628,8 @@ icx_status icx_basis_node_coords(const icx_ctx* ctx, double* xy);
  *               shared memory (the defaults there: 5 for FP32 factors, 4 for
  *               FP64 ones; at the default shape of 4 in FP64, and at every
  *               shape of 5 in FP32 and BF16, the factors are streamed through
- *               shared memory where the block size and the tile allow; each
+ *               shared memory where the block size and the tile allow and
+ *               that form is ahead; each
  *               falls back to the one below where its shared memory does not
  *               fit; 3 to 5 are 2 on whole-grid factors; 5 sums a row's
  *               columns in another order where it does not stream, so
