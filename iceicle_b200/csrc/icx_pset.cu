@@ -241,11 +241,10 @@ icx_status ensure_buffers(icx_pset* S, int m) {
   // the large ones: where memory is short, what the groups can do without is given back first
   const auto get = [&](double** p, size_t bytes) {
     cudaError_t e = cudaMalloc((void**)p, bytes);
-    for (size_t g = 0; g < S->groups.size() && e == cudaErrorMemoryAllocation; ++g) {
-      (void)cudaGetLastError();
+    for (size_t g = 0; g < S->groups.size() && e == cudaErrorMemoryAllocation; ++g)
       if (icx::solver_give_back(S->groups[g])) e = cudaMalloc((void**)p, bytes);
-    }
     if (e != cudaSuccess) *p = nullptr;
+    (void)cudaGetLastError();  // a refusal that was answered, or is returned, is not the next launch's
     return e;
   };
   PCK(get(&S->V, sizeof(double) * (m + 1) * n));
